@@ -27,6 +27,11 @@ int qmhd_solver_profile_step(qmhd_solver* solver, double* ms_by_phase, int n);
 /* Measured FP64 FMA throughput of the current device in TFLOP/s. */
 int qmhd_fp64_fma_peak(double* tflops);
 
+/* The stage kernels' reciprocal 1/x and inverse square root 1/sqrt(x) of n
+ * host values (normal numbers; positive for the root), 1 <= n <= 2^26, for
+ * checking their accuracy against correctly rounded values. */
+int qmhd_probe_roots(const double* x, long long n, double* reciprocal, double* inverse_sqrt);
+
 /* Tile hooks of a decomposed domain (quasar_b200/tiles.py), the pieces the
  * reference's distributed runtime keeps inside its solver
  * (src/distributed/mhd_runtime.cpp: dt and admissibility reduced over the

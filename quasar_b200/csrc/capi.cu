@@ -285,6 +285,30 @@ int qmhd_fp64_fma_peak(double* tflops) {
   });
 }
 
+int qmhd_probe_roots(const double* x, long long n, double* reciprocal, double* inverse_sqrt) {
+  return guarded([&] {
+    need(x);
+    need(reciprocal);
+    need(inverse_sqrt);
+    if (n < 1 || n > (1LL << 26))
+      throw std::invalid_argument("qmhd_probe_roots: need 1 <= n <= 2^26");
+    struct Buffer {
+      double* p = nullptr;
+      ~Buffer() { cudaFree(p); }
+    } d;
+    const size_t bytes = sizeof(double) * size_t(n);
+    auto ck = [](cudaError_t e) {
+      if (e != cudaSuccess) throw qb::CudaError(std::string("probe_roots: ") + cudaGetErrorString(e));
+    };
+    ck(cudaMalloc(&d.p, 3 * bytes));
+    ck(cudaMemcpy(d.p, x, bytes, cudaMemcpyHostToDevice));
+    qb::launch_probe_roots(d.p, n, d.p + n, d.p + 2 * n, nullptr);
+    ck(cudaGetLastError());
+    ck(cudaMemcpy(reciprocal, d.p + n, bytes, cudaMemcpyDeviceToHost));
+    ck(cudaMemcpy(inverse_sqrt, d.p + 2 * n, bytes, cudaMemcpyDeviceToHost));
+  });
+}
+
 // ---- batched instances (include/quasar_mhd_batch.h) ------------------------
 int qmhd_batch_create(const qmhd_config* configs, int n, qmhd_batch** out) {
   return guarded([&] {

@@ -1392,40 +1392,36 @@ __global__ void k_face_lists(Grid g, const unsigned char* flag, int* xlist, int*
 namespace {
 
 struct Spd {
-  double v, f;
+  double v, f2;
 };
 
-// One side's |v_n| and fast speed (mhd_reduce.hip:254-325), with one
+// One side's |v_n| and squared fast speed (mhd_reduce.hip:254-325), with one
 // reciprocal of rho.  The discriminant is formed as (a^2 - b^2)^2 + 4 a^2 b_t^2,
 // which equals the reference's (a^2 + b^2)^2 - 4 a^2 b_n^2 but has no
 // cancellation: where the reference's rounding is amplified to sqrt(eps) (a
 // degenerate fan, a == b_n with b_t == 0) this form stays accurate to a few
-// ulps, and elsewhere both agree to rounding.
+// ulps, and elsewhere both agree to rounding.  A non-finite component makes
+// the pressure fail its test (point_admissible_p).
 template <int DIR>
-__device__ Spd speed_parts(const St& s, double gamma) {
-  if (!(isfinite(s.rho) && s.rho > 0.0 && isfinite(s.mx) && isfinite(s.my) &&
-        isfinite(s.mz) && isfinite(s.E) && isfinite(s.bx) && isfinite(s.by) && isfinite(s.bz)))
-    return Spd{kInf, kInf};
-  const double ir = 1.0 / s.rho;
+__device__ __forceinline__ Spd speed_parts(const St& s, double gamma) {
+  const double ir = rcp_nr(s.rho);
   const double p = pressure_f(s, gamma, ir);
-  if (!(isfinite(p) && p > 0.0)) return Spd{kInf, kInf};
+  if (!point_admissible_p(s, p)) return Spd{kInf, kInf};
   const double bn = DIR == 0 ? s.bx : s.by, b1 = DIR == 0 ? s.by : s.bx;
   const double a2 = gamma * p * ir;
   const double bn2 = bn * bn * ir;
   const double bt2 = (b1 * b1 + s.bz * s.bz) * ir;
   const double d = a2 - (bn2 + bt2);
   const double disc = d * d + 4.0 * a2 * bt2;
-  const double fast = sqrt(0.5 * ((a2 + bn2 + bt2) + sqrt(disc)));
-  const double vel = fabs(DIR == 0 ? s.mx : s.my) * ir;
-  if (!(isfinite(vel) && isfinite(fast))) return Spd{kInf, kInf};
-  return Spd{vel, fast};
+  return Spd{fabs(DIR == 0 ? s.mx : s.my) * ir, 0.5 * ((a2 + bn2 + bt2) + sqrt_nr(disc))};
 }
 
 // Weighted face rate 0.5*alpha/h of one Riemann problem (mhd_reduce.hip:331-383).
 template <int DIR, int ORDER>
 __device__ __forceinline__ double face_rate(const St& l, const St& r, double gamma, double h) {
   const Spd a = speed_parts<DIR>(l, gamma), b = speed_parts<DIR>(r, gamma);
-  const double rate = ORDER <= 1 ? fmax(a.v + a.f, b.v + b.f) : fmax(a.v, b.v) + fmax(a.f, b.f);
+  const double rate = ORDER <= 1 ? fmax(a.v + sqrt_nr(a.f2), b.v + sqrt_nr(b.f2))
+                                 : fmax(a.v, b.v) + sqrt_nr(fmax(a.f2, b.f2));
   if (!(isfinite(rate) && rate >= 0.0)) return kInf;
   return div_by(rate * 0.5, h, pow2_recip(h));
 }
@@ -1665,7 +1661,7 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
   auto tr = [&](int t) { return DIR == 0 ? fy + t : fy; };
   auto tcl = [&](int t) { return DIR == 0 ? fx : fx + t; };
   St l{}, r{};
-  double irl = 1.0, irr = 1.0;
+  double irl = 1.0, irr = 1.0, prl = 0.0, prr = 0.0;
   bool ok = true;
   {
     double w[N];
@@ -1685,9 +1681,11 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
     }
     l = St{pl[0], pl[1], pl[2], pl[3], pl[4], pl[5], pl[6], pl[7]};
     r = St{pr[0], pr[1], pr[2], pr[3], pr[4], pr[5], pr[6], pr[7]};
-    irl = 1.0 / l.rho;
-    irr = 1.0 / r.rho;
-    ok = point_admissible_ir(l, gamma, irl) && point_admissible_ir(r, gamma, irr);
+    irl = rcp_nr(l.rho);
+    irr = rcp_nr(r.rho);
+    prl = pressure_f(l, gamma, irl);
+    prr = pressure_f(r, gamma, irr);
+    ok = point_admissible_p(l, prl) && point_admissible_p(r, prr);
   }
   auto centre = [&](bool left) {
     const int o = left ? 0 : 8, rr = tr(H), cc = tcl(H);
@@ -1706,12 +1704,14 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
   if (!group_ok) {
     l = centre(true);
     r = centre(false);
-    irl = 1.0 / l.rho;
-    irr = 1.0 / r.rho;
+    irl = rcp_nr(l.rho);
+    irr = rcp_nr(r.rho);
+    prl = pressure_f(l, gamma, irl);
+    prr = pressure_f(r, gamma, irr);
   }
   double fv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (solve) {
-    const Fx f = riemann<DIR>(l, r, kLF, gamma, irl, irr);
+    const Fx f = riemann<DIR>(l, r, kLF, gamma, irl, irr, prl, prr);
     fv[0] = f.rho; fv[1] = f.mx; fv[2] = f.my; fv[3] = f.mz;
     fv[4] = f.E;   fv[5] = f.bx; fv[6] = f.by; fv[7] = f.bz;
   }
@@ -1850,8 +1850,9 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
     l = St{a0.x, a0.y, a1.x, a1.y, a2.x, a2.y, a3.x, a3.y};
     r = St{b0.x, b0.y, b1.x, b1.y, b2.x, b2.y, b3.x, b3.y};
   }
-  double irl = 1.0 / l.rho, irr = 1.0 / r.rho;
-  const bool ok = point_admissible_ir(l, gamma, irl) && point_admissible_ir(r, gamma, irr);
+  double irl = rcp_nr(l.rho), irr = rcp_nr(r.rho);
+  double prl = pressure_f(l, gamma, irl), prr = pressure_f(r, gamma, irr);
+  const bool ok = point_admissible_p(l, prl) && point_admissible_p(r, prr);
   auto centre = [&](bool left) {
     const int o = left ? 0 : 8, sc = slot(H);
     return St{tile[o * PS + sc],       tile[(o + 1) * PS + sc], tile[(o + 2) * PS + sc],
@@ -1870,12 +1871,14 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
   if (!group_ok) {
     l = centre(true);
     r = centre(false);
-    irl = 1.0 / l.rho;
-    irr = 1.0 / r.rho;
+    irl = rcp_nr(l.rho);
+    irr = rcp_nr(r.rho);
+    prl = pressure_f(l, gamma, irl);
+    prr = pressure_f(r, gamma, irr);
   }
   double fv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (solve) {
-    const Fx f = riemann<DIR>(l, r, kLF, gamma, irl, irr);
+    const Fx f = riemann<DIR>(l, r, kLF, gamma, irl, irr, prl, prr);
     fv[0] = f.rho; fv[1] = f.mx; fv[2] = f.my; fv[3] = f.mz;
     fv[4] = f.E;   fv[5] = f.bx; fv[6] = f.by; fv[7] = f.bz;
   }
@@ -3236,6 +3239,17 @@ int exchange_blocks(long long n) {
   return (int)(b < 4 * 148 ? (b > 0 ? b : 1) : 4 * 148);
 }
 }  // namespace
+
+// y[k] = rcp_nr(x[k]), z[k] = rsqrt_nr(x[k]) (the accuracy test's hook).
+__global__ void k_probe_roots(const double* __restrict__ x, long long n, double* y, double* z) {
+  const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  y[k] = rcp_nr(x[k]);
+  z[k] = rsqrt_nr(x[k]);
+}
+void launch_probe_roots(const double* x, long long n, double* y, double* z, cudaStream_t s) {
+  if (n > 0) k_probe_roots<<<cdiv(n, 256), 256, 0, s>>>(x, n, y, z);
+}
 
 void launch_flag_nonfinite(const double* v, long long n, unsigned long long* bad, cudaStream_t s) {
   if (n <= 0) return;
