@@ -247,21 +247,11 @@ __device__ __forceinline__ St swap_xy(const St& v) {
   return r;
 }
 
-// Finite, rho>0, finite velocity, p>0 (mhd_reconstruct.hip:414-427).
-__device__ __forceinline__ bool recon_admissible(const St& s, double gamma) {
-  if (!(isfinite(s.rho) && s.rho > 0.0)) return false;
-  const double ir = 1.0 / s.rho;
-  const double p = pressure_f(s, gamma, ir);
-  if (!(isfinite(s.mx * ir) && isfinite(s.my * ir) && isfinite(s.mz * ir) && isfinite(p) &&
-        p > 0.0))
-    return false;
-  return isfinite(s.mx) && isfinite(s.my) && isfinite(s.mz) && isfinite(s.E) &&
-         isfinite(s.bx) && isfinite(s.by) && isfinite(s.bz);
-}
-// mhd_face_quadrature.hpp:68-76, with 1/rho supplied.  Every component
-// enters the pressure, so with rho finite and positive "p finite and
-// positive" already fails for any non-finite component (an infinite momentum
-// or field drives p to -inf, an infinite energy to +/-inf, a NaN to NaN): the
+// Admissibility of a face or point state (mhd_reconstruct.hip:414-427,
+// mhd_face_quadrature.hpp:68-76), with its pressure supplied.  Every component
+// enters the pressure, so with rho finite and positive "p finite and positive"
+// already fails for any non-finite component (an infinite momentum or field
+// drives p to -inf, an infinite energy to +/-inf, a NaN to NaN): the
 // reference's per-component finiteness tests are implied and not repeated,
 // the decision is the same.
 __device__ __forceinline__ bool point_admissible_p(const St& s, double p) {
@@ -272,6 +262,10 @@ __device__ __forceinline__ bool point_admissible_ir(const St& s, double gamma, d
 }
 __device__ __forceinline__ bool point_admissible(const St& s, double gamma) {
   return point_admissible_ir(s, gamma, rcp_nr(s.rho));
+}
+
+__device__ __forceinline__ bool recon_admissible(const St& s, double gamma) {
+  return point_admissible(s, gamma);
 }
 
 // ---- MP limiter: numerics/mp_limiter.hpp ---------------------------------
@@ -289,10 +283,7 @@ __device__ __forceinline__ double minmod4(double a, double b, double c, double d
 // mp_limiter.hpp:71-148.  `fired` is set when the candidate was changed.
 // The normalisations by the local variation and the curvature scale use one
 // reciprocal each instead of a division per term (rounding-level difference).
-// Not inlined: the warp-cooperative reconstruction calls it four times per
-// round, and one shared body instead of four inlined copies relieves its
-// instruction-fetch stalls (reconstruction 37.0 -> 35.5 ms per rotor 4096^2
-// MP7 step, 12.6 -> 11.3 on Orszag-Tang 2048^2 MP7; the state bit-identical).
+// One window at a time: the form the label pass uses, which needs `fired`.
 __device__ __noinline__ double mp_limit(double vl, double vm2, double vm1, double v0,
                                            double vp1, double vp2, bool& fired) {
   const double dmn = v0 - vm1;
@@ -355,6 +346,82 @@ __device__ __forceinline__ double mp_recon(const double* v, bool& fired) {
   const double vl = mp_interp_plain<W>(v);
   constexpr int o = W == 5 ? 0 : 1;
   return mp_limit(vl, v[o], v[o + 1], v[o + 2], v[o + 3], v[o + 4], fired);
+}
+
+// ---- both face states of one characteristic variable ----------------------
+// x with its sign flipped where the bit `s` (0 or 0x80000000) is set.
+__device__ __forceinline__ double flip_sign(double x, int s) {
+  return __hiloint2double(__double2hiint(x) ^ s, __double2loint(x));
+}
+// minmod4(4 p - q, 4 q - p, p, q): with m and M the smaller and larger of |p|
+// and |q|, and p, q of one sign, the smallest argument is min(m, 4 m - M)
+// (4 M - m >= 3 M), zero if that is negative.
+__device__ __forceinline__ double mp_curvature(double p, double q) {
+  const double P = fabs(p), Q = fabs(q);
+  const bool lt = P < Q;
+  const double m = lt ? P : Q, M = lt ? Q : P;
+  const double t = fma(4.0, m, -M);
+  const double r = t < m ? t : m;
+  const bool ok = (__double2hiint(p) ^ __double2hiint(q)) >= 0 && __double2hiint(r) >= 0;
+  return ok ? flip_sign(r, __double2hiint(p) & 0x80000000) : 0.0;
+}
+// One side of mp_limiter.hpp:71-148 in coordinates relative to its centre
+// sample and flipped so that the unlimited offset cc is positive: dpl = vp1 -
+// v0, dmn = v0 - vm1, md and lc the median and large-curvature offsets.  In
+// these coordinates the lower limit is <= 0 <= the upper limit, so only the
+// upper one, min(max(dpl, md), max(4 dmn, lc)) or zero, can bind; it is at
+// least minmod(dpl, 4 dmn), so the early accept never changes the value and
+// only its round-off form is tested, |cc| |cm| <= 1e-10 var^2.  Of var's
+// four terms the two differences suffice: |cc| or |cm| is the largest only
+// where cc or cm is within 1e-10 of zero relative to a difference, and there
+// the limited and the unlimited value agree to that.  Returns the limited
+// offset.  NaN offsets compare false and are returned.
+__device__ __forceinline__ double mp_side(double cc, double dpl, double dmn, double md,
+                                          double lc) {
+  const int s = __double2hiint(cc) & 0x80000000;
+  const double ac = fabs(cc);
+  const double d = flip_sign(dpl, s), ul = flip_sign(4.0 * dmn, s);
+  const double m = flip_sign(md, s), c = flip_sign(lc, s);
+  const double A = d > m ? d : m, B = ul > c ? ul : c;
+  double bound = A < B ? A : B;
+  bound = __double2hiint(bound) < 0 ? 0.0 : bound;
+  double mm = fabs(d) < fabs(ul) ? d : ul;
+  mm = (__double2hiint(d) ^ __double2hiint(ul)) < 0 ? 0.0 : mm;
+  const double P = ac * (ac - mm) * 1e10;
+  const int above = __double2hiint(fma(dmn, dmn, -P)) & __double2hiint(fma(dpl, dpl, -P));
+  return ac > bound && above < 0 ? flip_sign(bound, s) : cc;
+}
+// The MP5 / MP7 face values on both sides of the face between samples H and
+// H + 1 of c[0 .. 2H + 1] (mp_limiter.hpp:71-224 for the window and its
+// mirror image).  Everything is formed from the first differences, which
+// the two sides share, as are the second differences and the median's
+// curvature; the interpolation weights are those of mp_interp_plain summed
+// onto the differences.  63 FP64 instructions at MP7 for the pair, where two
+// separate windows took about 180 with four divisions.
+template <int W>
+__device__ __forceinline__ void mp_pair_limit(const double* c, double& wl, double& wr) {
+  constexpr int H = W / 2;
+  double d[W];
+#pragma unroll
+  for (int k = 0; k < W; ++k) d[k] = c[k + 1] - c[k];
+  double cl, cr;
+  if (W == 5) {
+    constexpr double q = 1.0 / 60.0;
+    cl = fma(24.0 * q, d[2], fma(-2.0 * q, d[0], fma(11.0 * q, d[1], (-3.0 * q) * d[3])));
+    cr = -fma(24.0 * q, d[2], fma(-2.0 * q, d[4], fma(11.0 * q, d[3], (-3.0 * q) * d[1])));
+  } else {
+    constexpr double q = 1.0 / 420.0;
+    cl = fma(180.0 * q, d[3], fma(79.0 * q, d[2], (-34.0 * q) * d[4])) +
+         fma(-22.0 * q, d[1], fma(3.0 * q, d[0], (4.0 * q) * d[5]));
+    cr = -(fma(180.0 * q, d[3], fma(79.0 * q, d[4], (-34.0 * q) * d[2])) +
+           fma(-22.0 * q, d[5], fma(3.0 * q, d[6], (4.0 * q) * d[1])));
+  }
+  const double dm = d[H - 1], d0 = d[H], dp = d[H + 1];
+  const double s1 = dm - d[H - 2], s2 = d0 - dm, s3 = dp - d0, s4 = d[H + 2] - dp;
+  const double ph = mp_curvature(s2, s3), hd = 0.5 * d0;
+  const double ml = mp_curvature(s2, s1), mr = mp_curvature(s3, s4);
+  wl = c[H] + mp_side(cl, d0, dm, fma(-0.5, ph, hd), fma(4.0 / 3.0, ml, 0.5 * dm));
+  wr = c[H + 1] + mp_side(cr, -d0, -dp, fma(-0.5, ph, -hd), fma(4.0 / 3.0, mr, -0.5 * dp));
 }
 
 // ---- HLLD: numerics/hlld_core.hpp ----------------------------------------

@@ -735,11 +735,13 @@ __device__ __forceinline__ void finish_face(const Grid& g, const StateP& u, cons
 //            projection, MP limiter on both sides, back-projection (lane =
 //            components r and r + 4)
 //   phase 3  lane = face: states, fallback chain, stores (finish_face)
-// Every value is formed by the same operations in the same order as
-// mp_pair_loop, so the two paths agree to the FMA contraction the compiler
-// picks for each expression.  Four lanes per face (not seven) because the
-// exchanged operands are read once per lane: each shared-memory load costs
-// one wavefront per half-warp whether or not the lanes share its address.
+// The pair's rows and columns are kept as their thermal / magnetic and
+// velocity parts (WavePair) and both face states of a wave come from one
+// limiter evaluation (mp_pair_limit): 225 -> 177 warp instructions a face,
+// 433 -> 326 us per 1024^2 MP7 launch.  The two paths agree to rounding.  Four
+// lanes per face (not seven) because the exchanged operands are read once
+// per lane: each shared-memory load costs one wavefront per half-warp whether
+// or not the lanes share its address.
 //
 // Per-warp shared memory (doubles): a face record [kRec][32] and eight group
 // buffers R[7][8] followed by delta[8][7], whose first 14 slots later hold
@@ -758,62 +760,55 @@ constexpr int kWarpReconDoubles = kRec * 32 + kGroups * kGrpDoubles;
 constexpr int kReconWarps = 4;
 constexpr size_t kReconWarpSmem = size_t(kReconWarps) * kWarpReconDoubles * sizeof(double);
 
-// L row and R column of wave k (k = 7: zeros) without branching on k: the
-// three families are formed side by side and selected, entry for entry the
-// products of wave_vectors and the sums of conserved_row_col.
-__device__ __forceinline__ void wave_lr(const Eg& e, int k, double* Lr, double* Rc) {
-  const double rho = e.rho;
-  const double s2 = kRs2, Nf = 0.5 * e.ia2;
-  // magnetosonic (k = 0, 2, 4, 6): fast for 0 and 6, slow for 2 and 4;
-  // the "minus" member of each pair is k < 3
-  const bool fs = (k == 0 || k == 6);
-  const bool neg = k < 3;
-  const double qf = e.cf * e.af * e.sbn, qs = e.cs * e.as * e.sbn;
-  const double Af = e.a * e.af * e.sr, As = e.a * e.as * e.sr;
-  const double al = fs ? e.af : e.as;
-  const double cc = fs ? e.cf : e.cs;
-  const double qq = fs ? qs : -qf;
-  const double AA = fs ? As : -Af;
-  const double ac = al * cc, qb1 = qq * e.b1, qb2 = qq * e.b2;
-  const double nac = Nf * al * cc, nq1 = Nf * qq * e.b1, nq2 = Nf * qq * e.b2;
-  // Alfven (k = 1, 5): the "minus" member is k = 1
-  const double t5 = e.sbn * e.b2 * s2 * e.sr, t6 = e.sbn * e.b1 * s2 * e.sr;
-  const double u5 = e.sbn * e.b2 * s2 * e.isr, u6 = e.sbn * e.b1 * s2 * e.isr;
-  const double ab2 = -e.b2 * s2, ab1 = e.b1 * s2;
-  const bool ms = (k & 1) == 0 && k != 7, alf = k == 1 || k == 5, ent = k == 3;
-  const bool k1 = k == 1;
-  double rp[7], lp[7];
-  rp[0] = ms ? rho * al : (ent ? 1.0 : 0.0);
-  rp[1] = ms ? (neg ? -ac : ac) : 0.0;
-  rp[2] = ms ? (neg ? qb1 : -qb1) : (alf ? ab2 : 0.0);
-  rp[3] = ms ? (neg ? qb2 : -qb2) : (alf ? ab1 : 0.0);
-  rp[4] = ms ? al * e.ra2 : 0.0;
-  rp[5] = ms ? AA * e.b1 : (alf ? (k1 ? -t5 : t5) : 0.0);
-  rp[6] = ms ? AA * e.b2 : (alf ? (k1 ? t6 : -t6) : 0.0);
-  lp[0] = ent ? 1.0 : 0.0;
-  lp[1] = ms ? (neg ? -nac : nac) : 0.0;
-  lp[2] = ms ? (neg ? nq1 : -nq1) : (alf ? ab2 : 0.0);
-  lp[3] = ms ? (neg ? nq2 : -nq2) : (alf ? ab1 : 0.0);
-  lp[4] = ms ? Nf * al * e.ir : (ent ? -e.ia2 : 0.0);
-  lp[5] = ms ? Nf * AA * e.b1 * e.ir : (alf ? (k1 ? -u5 : u5) : 0.0);
-  lp[6] = ms ? Nf * AA * e.b2 * e.ir : (alf ? (k1 ? u6 : -u6) : 0.0);
-  const double gv = e.gm1;
-  Lr[0] = (((lp[0] * 1.0 + lp[1] * (-e.vn * e.ir)) + lp[2] * (-e.vt1 * e.ir)) +
-           lp[3] * (-e.vt2 * e.ir)) + lp[4] * (gv * e.hv2);
-  Lr[1] = lp[1] * e.ir + lp[4] * (-gv * e.vn);
-  Lr[2] = lp[2] * e.ir + lp[4] * (-gv * e.vt1);
-  Lr[3] = lp[3] * e.ir + lp[4] * (-gv * e.vt2);
-  Lr[4] = lp[4] * gv;
-  Lr[5] = lp[4] * (-gv * e.bt1) + lp[5];
-  Lr[6] = lp[4] * (-gv * e.bt2) + lp[6];
-  Rc[0] = rp[0];
-  Rc[1] = e.vn * rp[0] + e.rho * rp[1];
-  Rc[2] = e.vt1 * rp[0] + e.rho * rp[2];
-  Rc[3] = e.vt2 * rp[0] + e.rho * rp[3];
-  Rc[4] = (((((e.hv2 * rp[0] + (e.rho * e.vn) * rp[1]) + (e.rho * e.vt1) * rp[2]) +
-             (e.rho * e.vt2) * rp[3]) + e.igm * rp[4]) + e.bt1 * rp[5]) + e.bt2 * rp[6];
-  Rc[5] = rp[5];
-  Rc[6] = rp[6];
+// The pair of waves r and 6 - r (r = 0 fast, 1 Alfven, 2 slow; r = 3 the
+// entropy wave alone) as its thermal / magnetic part and its velocity part:
+// the rows are L_r = T - V and L_(6-r) = T + V, the columns likewise (the
+// Alfven wave 1 with its overall sign reversed, which cancels between row and
+// column and leaves the limiter's odd function unchanged).  Entries as in
+// wave_vectors and conserved_row_col; V touches the momenta (and, in a row,
+// the density, in a column the energy) only.  Alfven vectors are the
+// magnetosonic ones with the transverse direction turned by 90 degrees.
+struct WavePair {
+  double lt[7], lv[4];  // row parts; lv: components 0-3
+  double rt[7], rv[4];  // column parts; rv: components 1-4
+};
+__device__ __forceinline__ void wave_pair(const Eg& e, int r, WavePair& w) {
+  const bool fast = r == 0, alf = r == 1, ent = r == 3, ms = !alf && !ent;
+  const double al = fast ? e.af : e.as, cc = fast ? e.cf : e.cs;
+  const double ax = fast ? e.as : e.af, cx = fast ? e.cs : e.cf;
+  const double sx = fast ? -e.sbn : e.sbn, Nf = 0.5 * e.ia2;
+  const double t1 = alf ? -e.b2 : e.b1, t2 = alf ? e.b1 : e.b2;
+  // transverse velocity and field amplitudes
+  const double qv = ms ? cx * ax * sx : (alf ? kRs2 : 0.0);
+  const double qb = ms ? (fast ? ax : -ax) * e.a * e.sr : (alf ? -e.sbn * kRs2 * e.sr : 0.0);
+  const double vn = ms ? al * cc : 0.0, v1 = qv * t1, v2 = qv * t2;
+  const double r0 = ms ? e.rho * al : (ent ? 1.0 : 0.0), rp = ms ? al * e.ra2 : 0.0;
+  const double r5 = qb * t1, r6 = qb * t2;
+  const double fl = (ms ? Nf : 1.0) * e.ir;
+  const double l1 = fl * vn, l2 = fl * v1, l3 = fl * v2;
+  w.lv[0] = -(l1 * e.vn + l2 * e.vt1 + l3 * e.vt2);
+  w.lv[1] = l1;
+  w.lv[2] = l2;
+  w.lv[3] = l3;
+  const double g = (ms ? fl * al : (ent ? -e.ia2 : 0.0)) * e.gm1;
+  w.lt[0] = g * e.hv2 + (ent ? 1.0 : 0.0);
+  w.lt[1] = -g * e.vn;
+  w.lt[2] = -g * e.vt1;
+  w.lt[3] = -g * e.vt2;
+  w.lt[4] = g;
+  w.lt[5] = fl * r5 - g * e.bt1;
+  w.lt[6] = fl * r6 - g * e.bt2;
+  w.rv[0] = e.rho * vn;
+  w.rv[1] = e.rho * v1;
+  w.rv[2] = e.rho * v2;
+  w.rv[3] = e.vn * w.rv[0] + e.vt1 * w.rv[1] + e.vt2 * w.rv[2];
+  w.rt[0] = r0;
+  w.rt[1] = e.vn * r0;
+  w.rt[2] = e.vt1 * r0;
+  w.rt[3] = e.vt2 * r0;
+  w.rt[4] = (e.hv2 * r0 + e.igm * rp) + (e.bt1 * r5 + e.bt2 * r6);
+  w.rt[5] = r5;
+  w.rt[6] = r6;
 }
 
 // One warp's 32 faces (lane = face; `valid` false for lanes without one).
@@ -858,18 +853,16 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
   const unsigned vmask = __ballot_sync(0xffffffffu, valid);
   // phase 2: eight faces per round, four lanes per face
   const int gi = int(lane >> 2), rl = int(lane & 3u);
-  const bool two = rl < 3;           // lanes 0-2: waves rl and 6 - rl; lane 3: wave 3
-  const int ka = rl, kb = 6 - rl;    // kb == ka on lane 3
   double* grp = ws + kRec * 32 + gi * kGrpDoubles;
   const double gm1 = gamma - 1.0, igm = 1.0 / gm1;
-  constexpr double kT2 = (1024.0 * kEps) * (1024.0 * kEps);
+  constexpr double kTol = 1024.0 * kEps;
 #pragma unroll 1
   for (int rd = 0; rd < 4; ++rd) {
     if (((vmask >> (8 * rd)) & 0xFFu) == 0u) continue;  // warp-uniform
     const int f = 8 * rd + gi;
     const bool on = (vmask >> f) & 1u;
     const long long kf = __shfl_sync(0xffffffffu, k0, f);
-    double La[7], Lb[7];
+    WavePair w;
     bool ok = true;
     if (on) {
       const double* r = rec + f;
@@ -893,48 +886,55 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
       e.ra2 = r[(kRecE + 13) * 32];
       e.hv2 = r[(kRecE + 14) * 32];
       e.ir = r[(kRecE + 15) * 32];
-      e.isr = r[(kRecE + 16) * 32];
       e.gm1 = gm1;
       e.igm = igm;
-      double Ra[7], Rb[7];
-      wave_lr(e, ka, La, Ra);
-      wave_lr(e, kb, Lb, Rb);
+      wave_pair(e, rl, w);
+      // columns 2 r (T part) and 2 r + 1 (V part); the entropy column is 6
+      double* col = grp + kGrpR + 2 * rl * kRS;
 #pragma unroll
-      for (int m = 0; m < 7; ++m) grp[kGrpR + ka * kRS + m] = Ra[m];
-      if (two) {
+      for (int m = 0; m < 7; ++m) col[m] = w.rt[m];
+      if (rl < 3) {
+        col[kRS] = 0.0;
 #pragma unroll
-        for (int m = 0; m < 7; ++m) grp[kGrpR + kb * kRS + m] = Rb[m];
+        for (int m = 0; m < 4; ++m) col[kRS + 1 + m] = w.rv[m];
+        col[kRS + 5] = 0.0;
+        col[kRS + 6] = 0.0;
       }
     }
     __syncwarp();
-    // L R = I within 1024 ulp (mhd_eigensystem.hpp:416-430): this lane's L
-    // rows against every R column; |d| <= 1024 eps tested as
-    // d^2 <= (1024 eps)^2
+    // L R = I within 1024 ulp (mhd_eigensystem.hpp:416-430): the four
+    // products of this lane's rows T -+ V with a pair's columns are A + D -+
+    // (B + C) and A - D +- (B - C), so both members of each are within the
+    // tolerance where the sum of the two magnitudes is
     if (on) {
 #pragma unroll
-      for (int jc = 0; jc < 7; ++jc) {
-        const double2* R2 = reinterpret_cast<const double2*>(grp + kGrpR + jc * kRS);
+      for (int q = 0; q < 4; ++q) {
+        const double2* R2 = reinterpret_cast<const double2*>(grp + kGrpR + 2 * q * kRS);
         const double2 p0 = R2[0], p1 = R2[1], p2 = R2[2], p3 = R2[3];
-        const double R7[7] = {p0.x, p0.y, p1.x, p1.y, p2.x, p2.y, p3.x};
-        double da = 0.0, db = 0.0;
-#pragma unroll
-        for (int m = 0; m < 7; ++m) {
-          da += La[m] * R7[m];
-          db += Lb[m] * R7[m];
+        const double A = fma(w.lt[0], p0.x, fma(w.lt[1], p0.y, fma(w.lt[2], p1.x, w.lt[3] * p1.y))) +
+                         fma(w.lt[4], p2.x, fma(w.lt[5], p2.y, w.lt[6] * p3.x));
+        const double C = fma(w.lv[0], p0.x, fma(w.lv[1], p0.y, fma(w.lv[2], p1.x, w.lv[3] * p1.y)));
+        const double one = q == rl ? 1.0 : 0.0;
+        if (q < 3) {
+          const double2 v0 = R2[4], v1 = R2[5], v2 = R2[6];
+          const double B = fma(w.lt[1], v0.y, fma(w.lt[2], v1.x, fma(w.lt[3], v1.y, w.lt[4] * v2.x)));
+          const double Dd = fma(w.lv[1], v0.y, fma(w.lv[2], v1.x, w.lv[3] * v1.y));
+          ok = ok && fabs((A - one) + Dd) + fabs(B + C) <= kTol && fabs(A - Dd) + fabs(B - C) <= kTol;
+        } else {
+          ok = ok && fabs(A - one) + fabs(C) <= kTol;
         }
-        const double ea = da - (ka == jc ? 1.0 : 0.0), eb = db - (kb == jc ? 1.0 : 0.0);
-        ok = ok && (ea * ea <= kT2) && (eb * eb <= kT2);
       }
     }
     const unsigned okm = __ballot_sync(0xffffffffu, ok);
     const bool usable = ((okm >> (gi * 4)) & 0xFu) == 0xFu;
     if (on && !usable) {
+      // identity rows and columns: wave r is component r, wave 6 - r
+      // component 6 - r (the T and V slots hold them unmixed)
+      double* col = grp + kGrpR + 2 * rl * kRS;
 #pragma unroll
-      for (int v = 0; v < 7; ++v) {
-        La[v] = v == ka ? 1.0 : 0.0;
-        Lb[v] = v == kb ? 1.0 : 0.0;
-        grp[kGrpR + ka * kRS + v] = v == ka ? 1.0 : 0.0;
-        if (two) grp[kGrpR + kb * kRS + v] = v == kb ? 1.0 : 0.0;
+      for (int m = 0; m < 7; ++m) {
+        col[m] = m == rl ? 1.0 : 0.0;
+        if (rl < 3) col[kRS + m] = m == 6 - rl ? 1.0 : 0.0;
       }
     }
     // stencil deltas in the canonical frame: lane rl loads cells rl, rl + 4
@@ -962,37 +962,36 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
     if (on) {
 #pragma unroll
       for (int sc = 0; sc < S; ++sc) {
-        double d7[7];
-#pragma unroll
-        for (int v = 0; v < 7; ++v) d7[v] = grp[kGrpD + sc * 7 + v];
-        double aa = 0.0, ab = 0.0;
-#pragma unroll
-        for (int v = 0; v < 7; ++v) {
-          aa += La[v] * d7[v];
-          ab += Lb[v] * d7[v];
+        const double* dd = grp + kGrpD + sc * 7;
+        if (usable) {
+          const double d0 = dd[0], d1 = dd[1], d2 = dd[2], d3 = dd[3];
+          const double t = fma(w.lt[0], d0, fma(w.lt[1], d1, fma(w.lt[2], d2, w.lt[3] * d3))) +
+                           fma(w.lt[4], dd[4], fma(w.lt[5], dd[5], w.lt[6] * dd[6]));
+          const double v = fma(w.lv[0], d0, fma(w.lv[1], d1, fma(w.lv[2], d2, w.lv[3] * d3)));
+          cha[sc] = t - v;
+          chb[sc] = t + v;
+        } else {
+          cha[sc] = dd[rl];
+          chb[sc] = dd[6 - rl];
         }
-        cha[sc] = aa;
-        chb[sc] = ab;
       }
     }
-    __syncwarp();  // the deltas are read; w overwrites them
-    // MP limiter on both sides of both waves
+    __syncwarp();  // the deltas are read; the face values overwrite them
+    // MP limiter on both sides of both waves; kept as the sum and the
+    // difference that multiply the pair's T and V columns
     if (on) {
-      double win[W];
-      bool fl;
-#pragma unroll
-      for (int sc = 0; sc < W; ++sc) win[sc] = cha[sc];
-      grp[kGrpW + ka] = mp_recon<W>(win, fl);
-#pragma unroll
-      for (int sc = 0; sc < W; ++sc) win[sc] = cha[W - sc];
-      grp[kGrpW + 7 + ka] = mp_recon<W>(win, fl);
-      if (two) {
-#pragma unroll
-        for (int sc = 0; sc < W; ++sc) win[sc] = chb[sc];
-        grp[kGrpW + kb] = mp_recon<W>(win, fl);
-#pragma unroll
-        for (int sc = 0; sc < W; ++sc) win[sc] = chb[W - sc];
-        grp[kGrpW + 7 + kb] = mp_recon<W>(win, fl);
+      double al, ar, bl, br;
+      mp_pair_limit<W>(cha, al, ar);
+      double* x = grp + kGrpW + 2 * rl;
+      if (rl < 3) {
+        mp_pair_limit<W>(chb, bl, br);
+        x[0] = usable ? al + bl : al;
+        x[1] = usable ? bl - al : bl;
+        x[7] = usable ? ar + br : ar;
+        x[8] = usable ? br - ar : br;
+      } else {
+        x[0] = al;
+        x[7] = ar;
       }
     }
     __syncwarp();
