@@ -395,7 +395,8 @@ __device__ __forceinline__ void set_normal_b(St& s, double v) {
 // (mhd_eigensystem.hpp:63-171), shared by all seven waves.
 struct Eg {
   double rho, sr, cf, cs, a, af, as, b1, b2, sbn, vn, vt1, vt2, bt1, bt2;
-  double ia2, ra2, gm1, hv2, ir, isr, igm;
+  double ia2, ra2, gm1, hv2, ir, igm;
+  bool sure;  // L R = I within the tolerance for certain (below)
 };
 constexpr double kRs2 = 0.7071067811865475;  // 1/sqrt(2) rounded
 
@@ -416,20 +417,23 @@ __device__ __forceinline__ Eg eig_scalars(const St& s, double gamma) {
   e.sr = sqrt(e.rho);
   e.bt1 = w.by;
   e.bt2 = w.bz;
-  double cax, ca;
+  double cax, ca, den, clip = 0.0;
   magnetosonic(e.rho, p, w.bx, w.by, w.bz, gamma, e.cf, e.cs, e.a, cax, ca);
   {
     const double sc = e.cf > 0.0 ? e.cf : 1.0;
     const double cfn = e.cf / sc, csn = e.cs / sc, an = e.a / sc;
-    const double den = sub(mul(cfn, cfn), mul(csn, csn));
+    den = sub(mul(cfn, cfn), mul(csn, csn));
     if (den <= mul(64.0 * kEps, add(mul(cfn, cfn), mul(csn, csn)))) {
       e.af = kRs2;
       e.as = kRs2;
+      den = 0.0;
     } else {
       const double af2 = sub(mul(an, an), mul(csn, csn)) / den;
       const double as2 = sub(mul(cfn, cfn), mul(an, an)) / den;
       e.af = sqrt(af2 < 0.0 ? 0.0 : af2);
       e.as = sqrt(as2 < 0.0 ? 0.0 : as2);
+      const double least = af2 < as2 ? af2 : as2;
+      clip = least < 0.0 ? -least : 0.0;
     }
   }
   {
@@ -454,8 +458,33 @@ __device__ __forceinline__ Eg eig_scalars(const St& s, double gamma) {
   e.gm1 = gamma - 1.0;
   e.hv2 = 0.5 * ((e.vn * e.vn + e.vt1 * e.vt1) + e.vt2 * e.vt2);
   e.ir = ir;
-  e.isr = 1.0 / e.sr;
   e.igm = 1.0 / e.gm1;
+  // A bound that shows the L R = I check to pass without forming it.  With
+  // k = c_f / a, M = (|v_n| + |v_t1| + |v_t2|) / a, b = (|B_t1| + |B_t2|) /
+  // (a sqrt(rho)), g = gamma - 1 and d = 1 - c_s^2 / c_f^2, every sum of
+  // magnitudes sum_m |L_im R_mj| is at most
+  //   S = max(rho, 1/rho) max(a, 1/a) F,
+  //   F = 3 + 3 k + 2 M + 1.5 k^2 + (1 + 4 g) k M + 2 g M^2 + 3 g b
+  // (term by term over the fast, slow, Alfven and entropy rows and columns).
+  // The rounding of the entries (at most six operations each side) and of the
+  // product is below 24 u S, u = eps / 2, in any order of summation.  The
+  // rounding of the normalisations moves af^2 + as^2 - 1, and with the factor
+  // k^2 the sum af^2 c_f^2 + as^2 c_s^2 = a^2, by less than 19 u / d, and a
+  // negative square set to zero by its size c (where c_f or c_s itself is off
+  // by rounding): together below 24 u k^2 (1 / d + c / (24 u)).  So S + k^2
+  // (1 / d + c / (24 u)) <= 80 keeps all of it, with 20 u for the constants,
+  // below 2048 u = 1024 eps.  Most faces of a flow near Mach one pass it; the
+  // others (strong scales, near-degenerate fans, high Mach numbers) take the
+  // check itself.  Reconstruction 7.6 -> 6.4 ms per step on a flow at 2048^2
+  // MP7, with the shared-memory strides of mp_faces_warp.
+  {
+    const double k = e.cf * ia, g = e.gm1;
+    const double M = (fabs(e.vn) + fabs(e.vt1) + fabs(e.vt2)) * ia;
+    const double b = (fabs(e.bt1) + fabs(e.bt2)) * (ia * e.sr * ir);
+    const double F = 3.0 + 3.0 * (k + g * b) + 1.5 * (k * k) + M * (2.0 + (1.0 + 4.0 * g) * k + 2.0 * g * M);
+    const double W = (e.rho > ir ? e.rho : ir) * (e.a > ia ? e.a : ia);
+    e.sure = (80.0 - W * F) * den >= k * k * fma(den * clip, 3.8e14, 1.0);
+  }
   return e;
 }
 
@@ -492,8 +521,9 @@ __device__ __forceinline__ void wave_vectors(const Eg& e, int k, double* lp, dou
     rp[6] = k == 1 ? e.sbn * e.b1 * s2 * e.sr : -e.sbn * e.b1 * s2 * e.sr;
     lp[2] = -e.b2 * s2;
     lp[3] = e.b1 * s2;
-    lp[5] = k == 1 ? -e.sbn * e.b2 * s2 * e.isr : e.sbn * e.b2 * s2 * e.isr;
-    lp[6] = k == 1 ? e.sbn * e.b1 * s2 * e.isr : -e.sbn * e.b1 * s2 * e.isr;
+    const double isr = e.sr * e.ir;
+    lp[5] = k == 1 ? -e.sbn * e.b2 * s2 * isr : e.sbn * e.b2 * s2 * isr;
+    lp[6] = k == 1 ? e.sbn * e.b1 * s2 * isr : -e.sbn * e.b1 * s2 * isr;
   } else if (k == 2 || k == 4) {
     rp[0] = rho * e.as;
     rp[1] = k == 2 ? -e.as * e.cs : e.as * e.cs;
@@ -743,20 +773,21 @@ __device__ __forceinline__ void finish_face(const Grid& g, const StateP& u, cons
 // per lane: each shared-memory load costs one wavefront per half-warp whether
 // or not the lanes share its address.
 //
-// Per-warp shared memory (doubles): a face record [kRec][32] and eight group
-// buffers R[7][8] followed by delta[8][7], whose first 14 slots later hold
-// the projected face values w[2][7].  The R columns are padded to eight
-// doubles so that the L R = I check reads them as 16-byte pairs (half the
-// load instructions of scalar reads: reconstruction went 39.9 -> 37.8 ms per
-// rotor 4096^2 MP7 step); the group stride of 114 doubles
-// puts the eight groups' 16-byte reads on distinct banks.  Padding the
-// stencil deltas the same way measured no faster.
+// Per-warp shared memory (doubles): a face record [kRec] rows of kRecS, and
+// eight group buffers.  A group holds the four pairs' columns, 12 doubles
+// apart (T components 0-6, V components 1-4 at offset 8), then the stencil
+// deltas [8][7], whose first 16 slots later hold the face values (left 0-6,
+// right 8-14).  The strides keep the exchange off common banks: 16-byte column
+// stores at 12 r + 100 g, delta stores at 7 c + 100 g and the transposed
+// back-projection stores at 36 v + f are conflict-free or two-way (with 8, 114
+// and 32 the stores took 184 wavefronts a round against 92, and the L1 data
+// pipe, the kernel's tightest resource, was 72% busy).
 constexpr int kRecC = 0;    // canonical reference state, 8 components
-constexpr int kRecE = 8;    // 17 eigen scalars, later dl[7] and dr[7]
-constexpr int kRec = 25;
-constexpr int kGrpR = 0, kRS = 8, kGrpD = 56, kGrpW = 56, kGrpDoubles = 114;
+constexpr int kRecE = 8;    // 16 eigen scalars, later dl[7] and dr[7]
+constexpr int kRec = 24, kRecS = 36;
+constexpr int kPair = 12, kPairV = 8, kGrpD = 44, kGrpW = 44, kGrpDoubles = 100;
 constexpr int kGroups = 8;
-constexpr int kWarpReconDoubles = kRec * 32 + kGroups * kGrpDoubles;
+constexpr int kWarpReconDoubles = kRec * kRecS + kGroups * kGrpDoubles;
 constexpr int kReconWarps = 4;
 constexpr size_t kReconWarpSmem = size_t(kReconWarps) * kWarpReconDoubles * sizeof(double);
 
@@ -823,6 +854,7 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
   const long long k0 = valid ? g.idx(i, j) : 0;
   double* rec = ws;
   // phase 1: reference state and eigen scalars of this lane's face
+  bool sure = true;
   if (valid) {
     const St cl = load_cell(u, k0 - step), cr = load_cell(u, k0);
     St ref;
@@ -837,23 +869,25 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
     const St c = rot<DIR>(ref);
     const Eg e = eig_scalars(c, gamma);
     double* r = rec + lane;
-    r[(kRecC + 0) * 32] = c.rho;
-    r[(kRecC + 1) * 32] = c.mx;
-    r[(kRecC + 2) * 32] = c.my;
-    r[(kRecC + 3) * 32] = c.mz;
-    r[(kRecC + 4) * 32] = c.E;
-    r[(kRecC + 5) * 32] = c.bx;
-    r[(kRecC + 6) * 32] = c.by;
-    r[(kRecC + 7) * 32] = c.bz;
-    const double ev[17] = {e.sr, e.cf, e.cs, e.a, e.af, e.as, e.b1, e.b2, e.sbn,
-                           e.vn, e.vt1, e.vt2, e.ia2, e.ra2, e.hv2, e.ir, e.isr};
+    r[(kRecC + 0) * kRecS] = c.rho;
+    r[(kRecC + 1) * kRecS] = c.mx;
+    r[(kRecC + 2) * kRecS] = c.my;
+    r[(kRecC + 3) * kRecS] = c.mz;
+    r[(kRecC + 4) * kRecS] = c.E;
+    r[(kRecC + 5) * kRecS] = c.bx;
+    r[(kRecC + 6) * kRecS] = c.by;
+    r[(kRecC + 7) * kRecS] = c.bz;
+    const double ev[16] = {e.sr, e.cf, e.cs, e.a, e.af, e.as, e.b1, e.b2, e.sbn,
+                           e.vn, e.vt1, e.vt2, e.ia2, e.ra2, e.hv2, e.ir};
+    sure = e.sure;
 #pragma unroll
-    for (int q = 0; q < 17; ++q) r[(kRecE + q) * 32] = ev[q];
+    for (int q = 0; q < 16; ++q) r[(kRecE + q) * kRecS] = ev[q];
   }
   const unsigned vmask = __ballot_sync(0xffffffffu, valid);
+  const unsigned smask = __ballot_sync(0xffffffffu, sure);
   // phase 2: eight faces per round, four lanes per face
   const int gi = int(lane >> 2), rl = int(lane & 3u);
-  double* grp = ws + kRec * 32 + gi * kGrpDoubles;
+  double* grp = ws + kRec * kRecS + gi * kGrpDoubles;
   const double gm1 = gamma - 1.0, igm = 1.0 / gm1;
   constexpr double kTol = 1024.0 * kEps;
 #pragma unroll 1
@@ -867,75 +901,68 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
     if (on) {
       const double* r = rec + f;
       Eg e;
-      e.rho = r[(kRecC + 0) * 32];
-      e.bt1 = r[(kRecC + 6) * 32];
-      e.bt2 = r[(kRecC + 7) * 32];
-      e.sr = r[(kRecE + 0) * 32];
-      e.cf = r[(kRecE + 1) * 32];
-      e.cs = r[(kRecE + 2) * 32];
-      e.a = r[(kRecE + 3) * 32];
-      e.af = r[(kRecE + 4) * 32];
-      e.as = r[(kRecE + 5) * 32];
-      e.b1 = r[(kRecE + 6) * 32];
-      e.b2 = r[(kRecE + 7) * 32];
-      e.sbn = r[(kRecE + 8) * 32];
-      e.vn = r[(kRecE + 9) * 32];
-      e.vt1 = r[(kRecE + 10) * 32];
-      e.vt2 = r[(kRecE + 11) * 32];
-      e.ia2 = r[(kRecE + 12) * 32];
-      e.ra2 = r[(kRecE + 13) * 32];
-      e.hv2 = r[(kRecE + 14) * 32];
-      e.ir = r[(kRecE + 15) * 32];
+      e.rho = r[(kRecC + 0) * kRecS];
+      e.bt1 = r[(kRecC + 6) * kRecS];
+      e.bt2 = r[(kRecC + 7) * kRecS];
+      e.sr = r[(kRecE + 0) * kRecS];
+      e.cf = r[(kRecE + 1) * kRecS];
+      e.cs = r[(kRecE + 2) * kRecS];
+      e.a = r[(kRecE + 3) * kRecS];
+      e.af = r[(kRecE + 4) * kRecS];
+      e.as = r[(kRecE + 5) * kRecS];
+      e.b1 = r[(kRecE + 6) * kRecS];
+      e.b2 = r[(kRecE + 7) * kRecS];
+      e.sbn = r[(kRecE + 8) * kRecS];
+      e.vn = r[(kRecE + 9) * kRecS];
+      e.vt1 = r[(kRecE + 10) * kRecS];
+      e.vt2 = r[(kRecE + 11) * kRecS];
+      e.ia2 = r[(kRecE + 12) * kRecS];
+      e.ra2 = r[(kRecE + 13) * kRecS];
+      e.hv2 = r[(kRecE + 14) * kRecS];
+      e.ir = r[(kRecE + 15) * kRecS];
       e.gm1 = gm1;
       e.igm = igm;
       wave_pair(e, rl, w);
-      // columns 2 r (T part) and 2 r + 1 (V part); the entropy column is 6
-      double* col = grp + kGrpR + 2 * rl * kRS;
-#pragma unroll
-      for (int m = 0; m < 7; ++m) col[m] = w.rt[m];
+      double2* col = reinterpret_cast<double2*>(grp + kPair * rl);
+      col[0] = make_double2(w.rt[0], w.rt[1]);
+      col[1] = make_double2(w.rt[2], w.rt[3]);
+      col[2] = make_double2(w.rt[4], w.rt[5]);
+      col[3] = make_double2(w.rt[6], 0.0);
       if (rl < 3) {
-        col[kRS] = 0.0;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) col[kRS + 1 + m] = w.rv[m];
-        col[kRS + 5] = 0.0;
-        col[kRS + 6] = 0.0;
+        col[4] = make_double2(w.rv[0], w.rv[1]);
+        col[5] = make_double2(w.rv[2], w.rv[3]);
       }
     }
     __syncwarp();
-    // L R = I within 1024 ulp (mhd_eigensystem.hpp:416-430): the four
-    // products of this lane's rows T -+ V with a pair's columns are A + D -+
-    // (B + C) and A - D +- (B - C), so both members of each are within the
-    // tolerance where the sum of the two magnitudes is
-    if (on) {
+    // L R = I within 1024 ulp (mhd_eigensystem.hpp:416-430), where no face of
+    // the round is known to pass it: the four products of this lane's rows
+    // T -+ V with a pair's columns are A + D -+ (B + C) and A - D +- (B - C), so
+    // both members of each are within the tolerance where the sum of the two
+    // magnitudes is
+    bool usable = true;
+    if (((smask >> (8 * rd)) & 0xFFu) != 0xFFu) {  // warp-uniform
+      bool ok = true;
+      if (on) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double2* R2 = reinterpret_cast<const double2*>(grp + kGrpR + 2 * q * kRS);
-        const double2 p0 = R2[0], p1 = R2[1], p2 = R2[2], p3 = R2[3];
-        const double A = fma(w.lt[0], p0.x, fma(w.lt[1], p0.y, fma(w.lt[2], p1.x, w.lt[3] * p1.y))) +
-                         fma(w.lt[4], p2.x, fma(w.lt[5], p2.y, w.lt[6] * p3.x));
-        const double C = fma(w.lv[0], p0.x, fma(w.lv[1], p0.y, fma(w.lv[2], p1.x, w.lv[3] * p1.y)));
-        const double one = q == rl ? 1.0 : 0.0;
-        if (q < 3) {
-          const double2 v0 = R2[4], v1 = R2[5], v2 = R2[6];
-          const double B = fma(w.lt[1], v0.y, fma(w.lt[2], v1.x, fma(w.lt[3], v1.y, w.lt[4] * v2.x)));
-          const double Dd = fma(w.lv[1], v0.y, fma(w.lv[2], v1.x, w.lv[3] * v1.y));
-          ok = ok && fabs((A - one) + Dd) + fabs(B + C) <= kTol && fabs(A - Dd) + fabs(B - C) <= kTol;
-        } else {
-          ok = ok && fabs(A - one) + fabs(C) <= kTol;
+        for (int q = 0; q < 4; ++q) {
+          const double2* R2 = reinterpret_cast<const double2*>(grp + kPair * q);
+          const double2 p0 = R2[0], p1 = R2[1], p2 = R2[2], p3 = R2[3];
+          const double A = fma(w.lt[0], p0.x, fma(w.lt[1], p0.y, fma(w.lt[2], p1.x, w.lt[3] * p1.y))) +
+                           fma(w.lt[4], p2.x, fma(w.lt[5], p2.y, w.lt[6] * p3.x));
+          const double C = fma(w.lv[0], p0.x, fma(w.lv[1], p0.y, fma(w.lv[2], p1.x, w.lv[3] * p1.y)));
+          const double one = q == rl ? 1.0 : 0.0;
+          if (q < 3) {
+            const double2 v0 = R2[4], v1 = R2[5];
+            const double B = fma(w.lt[1], v0.x, fma(w.lt[2], v0.y, fma(w.lt[3], v1.x, w.lt[4] * v1.y)));
+            const double Dd = fma(w.lv[1], v0.x, fma(w.lv[2], v0.y, w.lv[3] * v1.x));
+            ok = ok && fabs((A - one) + Dd) + fabs(B + C) <= kTol && fabs(A - Dd) + fabs(B - C) <= kTol;
+          } else {
+            ok = ok && fabs(A - one) + fabs(C) <= kTol;
+          }
         }
       }
-    }
-    const unsigned okm = __ballot_sync(0xffffffffu, ok);
-    const bool usable = ((okm >> (gi * 4)) & 0xFu) == 0xFu;
-    if (on && !usable) {
-      // identity rows and columns: wave r is component r, wave 6 - r
-      // component 6 - r (the T and V slots hold them unmixed)
-      double* col = grp + kGrpR + 2 * rl * kRS;
-#pragma unroll
-      for (int m = 0; m < 7; ++m) {
-        col[m] = m == rl ? 1.0 : 0.0;
-        if (rl < 3) col[kRS + m] = m == 6 - rl ? 1.0 : 0.0;
-      }
+      const unsigned okm = __ballot_sync(0xffffffffu, ok);
+      usable = ((okm >> (gi * 4)) & 0xFu) == 0xFu;
     }
     // stencil deltas in the canonical frame: lane rl loads cells rl, rl + 4
     if (on) {
@@ -946,13 +973,13 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
         if (sc < S) {
           const St d = rot<DIR>(load_cell(u, kf + (long long)(sc - 1 - H) * step));
           double* dd = grp + kGrpD + sc * 7;
-          dd[0] = d.rho - r[(kRecC + 0) * 32];
-          dd[1] = d.mx - r[(kRecC + 1) * 32];
-          dd[2] = d.my - r[(kRecC + 2) * 32];
-          dd[3] = d.mz - r[(kRecC + 3) * 32];
-          dd[4] = d.E - r[(kRecC + 4) * 32];
-          dd[5] = d.by - r[(kRecC + 6) * 32];
-          dd[6] = d.bz - r[(kRecC + 7) * 32];
+          dd[0] = d.rho - r[(kRecC + 0) * kRecS];
+          dd[1] = d.mx - r[(kRecC + 1) * kRecS];
+          dd[2] = d.my - r[(kRecC + 2) * kRecS];
+          dd[3] = d.mz - r[(kRecC + 3) * kRecS];
+          dd[4] = d.E - r[(kRecC + 4) * kRecS];
+          dd[5] = d.by - r[(kRecC + 6) * kRecS];
+          dd[6] = d.bz - r[(kRecC + 7) * kRecS];
         }
       }
     }
@@ -982,35 +1009,50 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
     if (on) {
       double al, ar, bl, br;
       mp_pair_limit<W>(cha, al, ar);
-      double* x = grp + kGrpW + 2 * rl;
-      if (rl < 3) {
-        mp_pair_limit<W>(chb, bl, br);
-        x[0] = usable ? al + bl : al;
-        x[1] = usable ? bl - al : bl;
-        x[7] = usable ? ar + br : ar;
-        x[8] = usable ? br - ar : br;
-      } else {
-        x[0] = al;
-        x[7] = ar;
-      }
+      if (rl < 3) mp_pair_limit<W>(chb, bl, br);
+      else bl = br = 0.0;
+      // (without usable eigenvectors wave r is component r and wave 6 - r
+      // component 6 - r, kept unmixed)
+      double2* x = reinterpret_cast<double2*>(grp + kGrpW + 2 * rl);
+      x[0] = usable ? make_double2(al + bl, bl - al) : make_double2(al, bl);
+      x[4] = usable ? make_double2(ar + br, br - ar) : make_double2(ar, br);
     }
     __syncwarp();
     // back-projection: lane rl forms components rl and rl + 4 of both sides
     if (on) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int v = rl + 4 * h;
-        if (v < 7) {
-          double dl = 0.0, dr = 0.0;
-#pragma unroll
-          for (int q = 0; q < 7; ++q) {
-            const double rq = grp[kGrpR + q * kRS + v];
-            dl += rq * grp[kGrpW + q];
-            dr += rq * grp[kGrpW + 7 + q];
-          }
-          rec[(kRecE + v) * 32 + f] = dl;
-          rec[(kRecE + 7 + v) * 32 + f] = dr;
+      const double2* x2 = reinterpret_cast<const double2*>(grp + kGrpW);
+      const double2 l0 = x2[0], l1 = x2[1], l2 = x2[2], l3 = x2[3];
+      const double2 r0 = x2[4], r1 = x2[5], r2 = x2[6], r3 = x2[7];
+      const int v1 = rl > 0 ? kPairV + rl - 1 : 7;  // V part of component rl (7: a zero)
+      const double t0 = grp[rl], t1 = grp[kPair + rl], t2 = grp[2 * kPair + rl], t3 = grp[3 * kPair + rl];
+      const double u0 = grp[v1], u1 = grp[kPair + v1], u2 = grp[2 * kPair + v1];
+      double dl = fma(t0, l0.x, fma(t1, l1.x, fma(t2, l2.x, t3 * l3.x))) +
+                  fma(u0, l0.y, fma(u1, l1.y, u2 * l2.y));
+      double dr = fma(t0, r0.x, fma(t1, r1.x, fma(t2, r2.x, t3 * r3.x))) +
+                  fma(u0, r0.y, fma(u1, r1.y, u2 * r2.y));
+      if (!usable) {
+        dl = rl == 0 ? l0.x : rl == 1 ? l1.x : rl == 2 ? l2.x : l3.x;
+        dr = rl == 0 ? r0.x : rl == 1 ? r1.x : rl == 2 ? r2.x : r3.x;
+      }
+      rec[(kRecE + rl) * kRecS + f] = dl;
+      rec[(kRecE + 7 + rl) * kRecS + f] = dr;
+      if (rl < 3) {  // components 4, 5, 6; of these only the energy has a V part
+        const double s0 = grp[rl + 4], s1 = grp[kPair + rl + 4], s2 = grp[2 * kPair + rl + 4],
+                     s3 = grp[3 * kPair + rl + 4];
+        double el = fma(s0, l0.x, fma(s1, l1.x, fma(s2, l2.x, s3 * l3.x)));
+        double er = fma(s0, r0.x, fma(s1, r1.x, fma(s2, r2.x, s3 * r3.x)));
+        if (rl == 0) {
+          const double w0 = grp[kPairV + 3], w1 = grp[kPair + kPairV + 3],
+                       w2 = grp[2 * kPair + kPairV + 3];
+          el += fma(w0, l0.y, fma(w1, l1.y, w2 * l2.y));
+          er += fma(w0, r0.y, fma(w1, r1.y, w2 * r2.y));
         }
+        if (!usable) {
+          el = rl == 0 ? l2.y : rl == 1 ? l1.y : l0.y;
+          er = rl == 0 ? r2.y : rl == 1 ? r1.y : r0.y;
+        }
+        rec[(kRecE + 4 + rl) * kRecS + f] = el;
+        rec[(kRecE + 11 + rl) * kRecS + f] = er;
       }
     }
     __syncwarp();
@@ -1019,19 +1061,19 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
   if (!valid) return;
   const double* r = rec + lane;
   St c;
-  c.rho = r[(kRecC + 0) * 32];
-  c.mx = r[(kRecC + 1) * 32];
-  c.my = r[(kRecC + 2) * 32];
-  c.mz = r[(kRecC + 3) * 32];
-  c.E = r[(kRecC + 4) * 32];
-  c.bx = r[(kRecC + 5) * 32];
-  c.by = r[(kRecC + 6) * 32];
-  c.bz = r[(kRecC + 7) * 32];
+  c.rho = r[(kRecC + 0) * kRecS];
+  c.mx = r[(kRecC + 1) * kRecS];
+  c.my = r[(kRecC + 2) * kRecS];
+  c.mz = r[(kRecC + 3) * kRecS];
+  c.E = r[(kRecC + 4) * kRecS];
+  c.bx = r[(kRecC + 5) * kRecS];
+  c.by = r[(kRecC + 6) * kRecS];
+  c.bz = r[(kRecC + 7) * kRecS];
   double dl[7], dr[7];
 #pragma unroll
   for (int v = 0; v < 7; ++v) {
-    dl[v] = r[(kRecE + v) * 32];
-    dr[v] = r[(kRecE + 7 + v) * 32];
+    dl[v] = r[(kRecE + v) * kRecS];
+    dr[v] = r[(kRecE + 7 + v) * kRecS];
   }
   const St sl{c.rho + dl[0], c.mx + dl[1], c.my + dl[2], c.mz + dl[3],
               c.E + dl[4],   c.bx,         c.by + dl[5], c.bz + dl[6]};
