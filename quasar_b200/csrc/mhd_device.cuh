@@ -205,29 +205,20 @@ __device__ __forceinline__ double fast_x_f(const St& u, double p, double ir, dou
   return sqrt(0.5 * ((a2 + bn2 + bt2) + sqrt(disc)));
 }
 
+// Conserved <-> primitive for the limited slopes of the second-order faces,
+// whose result depends continuously on rounding: plain arithmetic with one
+// reciprocal of rho (igm = 1 / (gamma - 1)) instead of the component-scaled
+// forms' seven divisions a state.
 __device__ __forceinline__ Pr to_prim(const St& u, double gamma) {
-  Pr w;
-  w.rho = u.rho;
-  w.vx = u.mx / u.rho;
-  w.vy = u.my / u.rho;
-  w.vz = u.mz / u.rho;
-  w.bx = u.bx;
-  w.by = u.by;
-  w.bz = u.bz;
-  w.p = pressure(u, gamma);
-  return w;
+  const double ir = rcp_nr(u.rho);
+  return Pr{u.rho, u.mx * ir, u.my * ir, u.mz * ir, pressure_f(u, gamma, ir), u.bx, u.by, u.bz};
 }
-__device__ __forceinline__ St to_cons(const Pr& w, double gamma) {
-  St u;
-  u.rho = w.rho;
-  u.mx = w.rho * w.vx;
-  u.my = w.rho * w.vy;
-  u.mz = w.rho * w.vz;
-  u.bx = w.bx;
-  u.by = w.by;
-  u.bz = w.bz;
-  u.E = w.p / (gamma - 1.0) + kin_vel(w.rho, w.vx, w.vy, w.vz) + half_sq3(w.bx, w.by, w.bz);
-  return u;
+__device__ __forceinline__ St to_cons(const Pr& w, double igm) {
+  const double mx = w.rho * w.vx, my = w.rho * w.vy, mz = w.rho * w.vz;
+  return St{w.rho, mx, my, mz,
+            w.p * igm + 0.5 * (mx * w.vx + my * w.vy + mz * w.vz) +
+                0.5 * (w.bx * w.bx + w.by * w.by + w.bz * w.bz),
+            w.bx, w.by, w.bz};
 }
 // mhd_state.hpp:272-289 (x-normal)
 __device__ __forceinline__ double fast_x(const St& u, double gamma) {

@@ -1117,8 +1117,9 @@ __device__ void muscl_pair(const Grid& g, const StateP& u, int i, int j, long lo
   const int n = DIR == 0 ? g.nx : g.ny;
   const int lo = g.bc[DIR * 2], hi = g.bc[DIR * 2 + 1];
   const int pos = DIR == 0 ? i : j;
-  ul = to_cons(muscl_face(a, b, c, 1.0, slope_drop(pos - 1, n, lo, hi)), gamma);
-  ur = to_cons(muscl_face(b, c, d, -1.0, slope_drop(pos, n, lo, hi)), gamma);
+  const double igm = 1.0 / (gamma - 1.0);
+  ul = to_cons(muscl_face(a, b, c, 1.0, slope_drop(pos - 1, n, lo, hi)), igm);
+  ur = to_cons(muscl_face(b, c, d, -1.0, slope_drop(pos, n, lo, hi)), igm);
 }
 
 // How far the limited characteristic face state departs from the unlimited
@@ -3181,9 +3182,11 @@ void launch_update(const StageArgs& a, const StateP& un, const StateP& us, const
                    int stage, const double* dt_dev, double dt_host, cudaStream_t s) {
   const Grid& g = a.g;
   const dim3 block(kBX, 8);
-  // the paired form needs an even pitch, at least three ghost layers and
-  // 16-byte aligned arrays
-  bool pairs = (g.pitch % 2) == 0 && g.ng >= 3;
+  // the paired form needs an even pitch, 16-byte aligned arrays and two ghost
+  // layers (a pair's partner reads stay inside the padded arrays: at most two
+  // columns past the last face, in a row before the last).  MUSCL 1024^2:
+  // update 0.263 -> 0.184 ms per step.
+  bool pairs = (g.pitch % 2) == 0 && g.ng >= 2;
   auto al = [](const double* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   for (int q = 0; q < 8 && pairs; ++q)
     pairs = al(un.c[q]) && al(us.c[q]) && al(out.c[q]) && al(a.fx.f[q]) && al(a.fy.f[q]);
