@@ -1641,6 +1641,34 @@ constexpr int kFqRow = 18;
 template <int ORDER>
 constexpr int fq_face() { return (ORDER == 5 ? 3 : 4) * kFqRow + 4; }
 
+// All 2H + 1 transverse taps of a face staged with L == R in every component,
+// from the tile's bits: the taps are N consecutive slots from s0 (y faces) or
+// every TC-th one (x faces).
+template <int DIR, int N>
+__device__ __forceinline__ bool stencil_flat(const unsigned* same, int s0, int TC) {
+  if (DIR == 1) {
+    const unsigned b = __funnelshift_r(same[s0 >> 5], same[(s0 >> 5) + 1], s0 & 31);
+    return (b & ((1u << N) - 1u)) == (1u << N) - 1u;
+  }
+  unsigned all = 1u;
+#pragma unroll
+  for (int t = 0; t < N; ++t) all &= same[(s0 + t * TC) >> 5] >> ((s0 + t * TC) & 31);
+  return all & 1u;
+}
+// Flux of a point whose two sides are the same state: the physical flux.
+template <int DIR>
+__device__ __forceinline__ Fx flat_flux(const St& s, double p, double ir) {
+  Fx f = physical_flux_xp(rot<DIR>(s), p, ir);
+  if (DIR == 1) {
+    const double t = f.mx;
+    f.mx = f.my;
+    f.my = t;
+    f.bx = f.by;
+    f.by = 0.0;
+  }
+  return f;
+}
+
 // Per-point recovery (MP5): each lane forms all 16 components of its own
 // Gauss point from the staged tile, and the group gathers the point fluxes
 // by shuffles.  With three lanes per face the component split below leaves
@@ -1656,11 +1684,15 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
   constexpr int TR = DIR == 0 ? TY + 2 * H : TY;          // tile rows (j)
   constexpr int TC = DIR == 0 ? TX : TX + 2 * H;          // tile columns (i)
   __shared__ double tile[16][TR][TC];
-  __shared__ unsigned char same[TR][TC];  // staged and L == R in every component
+  // staged and L == R in every component: one bit per tile slot
+  constexpr int kWords = (TR * TC + 31) / 32;
+  __shared__ unsigned same[kWords + 1];
   if (ctl->status) return;  // uniform over the block
   const int i0 = bx * TX, j0 = by * TY;
   const bool perx = g.bc[0] == 0 && g.bc[1] == 0, pery = g.bc[2] == 0 && g.bc[3] == 0;
-  for (int e = threadIdx.x; e < TR * TC; e += blockDim.x) {
+  static_assert(TR * TC <= kFqThreads, "one tile slot per thread");
+  {
+    const int e = threadIdx.x;
     const int row = e / TC, col = e - row * TC;
     int fi, fj;
     bool valid;
@@ -1668,12 +1700,12 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
       const int ii = i0 + col;
       fi = (ii == g.nx && perx) ? 0 : ii;
       fj = j0 - H + row;
-      valid = ii <= g.nx && fj >= -g.ng && fj < g.ny + g.ng;
+      valid = e < TR * TC && ii <= g.nx && fj >= -g.ng && fj < g.ny + g.ng;
     } else {
       const int jj = j0 + row;
       fj = (jj == g.ny && pery) ? 0 : jj;
       fi = i0 - H + col;
-      valid = jj <= g.ny && fi >= -g.ng && fi < g.nx + g.ng;
+      valid = e < TR * TC && jj <= g.ny && fi >= -g.ng && fi < g.nx + g.ng;
     }
     const long long kk = valid ? g.idx(fi, fj) : 0;
     bool eq = valid;
@@ -1681,11 +1713,15 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
     for (int c = 0; c < 8; ++c) {
       const double a = valid ? __ldg(in.L[c] + kk) : 0.0;
       const double b = valid ? __ldg(in.R[c] + kk) : 0.0;
-      tile[c][row][col] = a;
-      tile[8 + c][row][col] = b;
+      if (e < TR * TC) {
+        tile[c][row][col] = a;
+        tile[8 + c][row][col] = b;
+      }
       eq = eq && a == b;
     }
-    same[row][col] = eq;
+    const unsigned w = __ballot_sync(0xffffffffu, eq);
+    if ((e & 31) == 0 && e / 32 < kWords) same[e / 32] = w;
+    if (e == 0) same[kWords] = 0u;
   }
   __syncthreads();
   constexpr bool kLF = false;
@@ -1702,6 +1738,8 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
   // tile coordinates of stencil tap t (t = H is the face itself)
   auto tr = [&](int t) { return DIR == 0 ? fy + t : fy; };
   auto tcl = [&](int t) { return DIR == 0 ? fx : fx + t; };
+  auto slot = [&](int t) { return tr(t) * TC + tcl(t); };
+  const bool flat = stencil_flat<DIR, N>(same, slot(0), TC);
   St l{}, r{};
   double irl = 1.0, irr = 1.0, prl = 0.0, prr = 0.0;
   bool ok = true;
@@ -1753,7 +1791,7 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
   }
   double fv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (solve) {
-    const Fx f = riemann<DIR>(l, r, kLF, gamma, irl, irr, prl, prr);
+    const Fx f = flat ? flat_flux<DIR>(l, prl, irl) : riemann<DIR, false>(l, r, kLF, gamma, irl, irr, prl, prr);
     fv[0] = f.rho; fv[1] = f.mx; fv[2] = f.my; fv[3] = f.mz;
     fv[4] = f.E;   fv[5] = f.bx; fv[6] = f.by; fv[7] = f.bz;
   }
@@ -1785,9 +1823,12 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
     if (lane == 0) spd[k] = m;
   }
   if (!nj) return;  // uniform over the block
-  // no-jump proof over the 2H+1 transverse taps (mapped like every CT table
-  // read), split across the group.  A tap whose mapped face is the one staged
-  // in its tile slot reads the staged comparison; the others read memory.
+  // no-jump proof (as in b_face_flux_cs)
+  const bool inner = DIR == 0 ? (j0 >= H && j0 + TY - 1 + H < g.ny) : (i0 >= H && i0 + TX - 1 + H < g.nx);
+  if (inner) {
+    if (lane == 0) nj[k] = flat ? 1 : 0;
+    return;
+  }
   int proof = 1;
   for (int off = lane - H; off <= H; off += Q) {
     const int mi = face_index(DIR == 0 ? i : i + off, g.nx, g.bc[0], g.bc[1]);
@@ -1795,7 +1836,8 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
     const int ti = DIR == 0 ? ((i == g.nx && perx) ? 0 : i) : i + off;
     const int tj = DIR == 0 ? j + off : ((j == g.ny && pery) ? 0 : j);
     if (mi == ti && mj == tj) {
-      if (!same[tr(off + H)][tcl(off + H)]) proof = 0;
+      const int sl = slot(off + H);
+      if (!(same[sl >> 5] >> (sl & 31) & 1u)) proof = 0;
       continue;
     }
     if (!in_pad(g, mi, mj)) {
@@ -1823,12 +1865,16 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
   constexpr int TC = DIR == 0 ? TX : TX + 2 * H;          // tile columns (i)
   constexpr int PS = fq_plane(TR * TC), FS = fq_face<ORDER>();
   __shared__ double tile[16 * PS];             // component c of slot (row, col): c PS + row TC + col
-  __shared__ unsigned char same[TR][TC];       // staged and L == R in every component
+  // staged and L == R in every component: one bit per tile slot
+  constexpr int kWords = (TR * TC + 31) / 32;
+  __shared__ unsigned same[kWords + 1];
   __shared__ __align__(16) double pts[4 * FPW * FS];  // per face: Q point rows
   if (ctl->status) return;  // uniform over the block
   const int i0 = bx * TX, j0 = by * TY;
   const bool perx = g.bc[0] == 0 && g.bc[1] == 0, pery = g.bc[2] == 0 && g.bc[3] == 0;
-  for (int e = threadIdx.x; e < TR * TC; e += blockDim.x) {
+  static_assert(TR * TC <= kFqThreads, "one tile slot per thread");
+  {
+    const int e = threadIdx.x;
     const int row = e / TC, col = e - row * TC;
     int fi, fj;
     bool valid;
@@ -1836,12 +1882,12 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
       const int ii = i0 + col;
       fi = (ii == g.nx && perx) ? 0 : ii;
       fj = j0 - H + row;
-      valid = ii <= g.nx && fj >= -g.ng && fj < g.ny + g.ng;
+      valid = e < TR * TC && ii <= g.nx && fj >= -g.ng && fj < g.ny + g.ng;
     } else {
       const int jj = j0 + row;
       fj = (jj == g.ny && pery) ? 0 : jj;
       fi = i0 - H + col;
-      valid = jj <= g.ny && fi >= -g.ng && fi < g.nx + g.ng;
+      valid = e < TR * TC && jj <= g.ny && fi >= -g.ng && fi < g.nx + g.ng;
     }
     const long long kk = valid ? g.idx(fi, fj) : 0;
     bool eq = valid;
@@ -1849,16 +1895,20 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
     for (int c = 0; c < 8; ++c) {
       const double a = valid ? __ldg(in.L[c] + kk) : 0.0;
       const double b = valid ? __ldg(in.R[c] + kk) : 0.0;
-      tile[c * PS + e] = a;
-      tile[(8 + c) * PS + e] = b;
+      if (e < TR * TC) {
+        tile[c * PS + e] = a;
+        tile[(8 + c) * PS + e] = b;
+      }
       eq = eq && a == b;
     }
-    same[row][col] = eq;
+    const unsigned w = __ballot_sync(0xffffffffu, eq);
+    if ((e & 31) == 0 && e / 32 < kWords) same[e / 32] = w;
+    if (e == 0) same[kWords] = 0u;
   }
   __syncthreads();
   constexpr bool kLF = false;
   const int wl = threadIdx.x & 31;
-  if (wl >= FPW * Q) return;  // the lanes no group uses (MP5)
+  static_assert(FPW * Q == 32, "every lane has a group");
   const int lane = wl % Q, base = wl - lane;
   const unsigned gmask = ((1u << Q) - 1u) << base;
   const int face = (threadIdx.x >> 5) * FPW + wl / Q;
@@ -1870,6 +1920,7 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
   // tile slot of stencil tap t (t = H is the face itself)
   auto slot = [&](int t) { return DIR == 0 ? (fy + t) * TC + fx : fy * TC + fx + t; };
   double* const fp = pts + face * FS;  // this face's point rows
+  const bool flat = stencil_flat<DIR, N>(same, slot(0), TC);
   // point values of components lane, lane + Q, ... at the Q Gauss nodes
 #pragma unroll
   for (int m = 0; m < (16 + Q - 1) / Q; ++m) {
@@ -1920,7 +1971,7 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
   }
   double fv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (solve) {
-    const Fx f = riemann<DIR>(l, r, kLF, gamma, irl, irr, prl, prr);
+    const Fx f = flat ? flat_flux<DIR>(l, prl, irl) : riemann<DIR, false>(l, r, kLF, gamma, irl, irr, prl, prr);
     fv[0] = f.rho; fv[1] = f.mx; fv[2] = f.my; fv[3] = f.mz;
     fv[4] = f.E;   fv[5] = f.bx; fv[6] = f.by; fv[7] = f.bz;
   }
@@ -1971,8 +2022,15 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
   }
   if (!nj) return;  // uniform over the block
   // no-jump proof over the 2H+1 transverse taps (mapped like every CT table
-  // read), split across the group.  A tap whose mapped face is the one staged
-  // in its tile slot reads the staged comparison; the others read memory.
+  // read).  Where no tap of the tile is mapped, the staged bits are the proof
+  // (a block-uniform test; the general form below is about 100 instructions).
+  const bool inner = DIR == 0 ? (j0 >= H && j0 + TY - 1 + H < g.ny) : (i0 >= H && i0 + TX - 1 + H < g.nx);
+  if (inner) {
+    if (lane == 0) nj[k] = flat ? 1 : 0;
+    return;
+  }
+  // the group splits the taps; one whose mapped face is the one staged in its
+  // tile slot reads the staged bit, the others read memory
   int proof = 1;
   for (int off = lane - H; off <= H; off += Q) {
     const int mi = face_index(DIR == 0 ? i : i + off, g.nx, g.bc[0], g.bc[1]);
@@ -1981,7 +2039,7 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
     const int tj = DIR == 0 ? j + off : ((j == g.ny && pery) ? 0 : j);
     if (mi == ti && mj == tj) {
       const int sl = slot(off + H);
-      if (!same[sl / TC][sl % TC]) proof = 0;
+      if (!(same[sl >> 5] >> (sl & 31) & 1u)) proof = 0;
       continue;
     }
     if (!in_pad(g, mi, mj)) {
