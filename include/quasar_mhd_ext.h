@@ -32,6 +32,10 @@ int qmhd_fp64_fma_peak(double* tflops);
  * checking their accuracy against correctly rounded values. */
 int qmhd_probe_roots(const double* x, long long n, double* reciprocal, double* inverse_sqrt);
 
+/* a[k] / b[k] of n host pairs as the reconstruction's eigen scalars divide,
+ * for checking that the bits are those of IEEE division. */
+int qmhd_probe_quotients(const double* a, const double* b, long long n, double* quotient);
+
 /* Tile hooks of a decomposed domain (quasar_b200/tiles.py), the pieces the
  * reference's distributed runtime keeps inside its solver
  * (src/distributed/mhd_runtime.cpp: dt and admissibility reduced over the

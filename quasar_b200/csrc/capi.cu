@@ -309,6 +309,31 @@ int qmhd_probe_roots(const double* x, long long n, double* reciprocal, double* i
   });
 }
 
+int qmhd_probe_quotients(const double* a, const double* b, long long n, double* quotient) {
+  return guarded([&] {
+    need(a);
+    need(b);
+    need(quotient);
+    if (n < 1 || n > (1LL << 26))
+      throw std::invalid_argument("qmhd_probe_quotients: need 1 <= n <= 2^26");
+    struct Buffer {
+      double* p = nullptr;
+      ~Buffer() { cudaFree(p); }
+    } d;
+    const size_t bytes = sizeof(double) * size_t(n);
+    auto ck = [](cudaError_t e) {
+      if (e != cudaSuccess)
+        throw qb::CudaError(std::string("probe_quotients: ") + cudaGetErrorString(e));
+    };
+    ck(cudaMalloc(&d.p, 3 * bytes));
+    ck(cudaMemcpy(d.p, a, bytes, cudaMemcpyHostToDevice));
+    ck(cudaMemcpy(d.p + n, b, bytes, cudaMemcpyHostToDevice));
+    qb::launch_probe_quotients(d.p, d.p + n, n, d.p + 2 * n, nullptr);
+    ck(cudaGetLastError());
+    ck(cudaMemcpy(quotient, d.p + 2 * n, bytes, cudaMemcpyDeviceToHost));
+  });
+}
+
 // ---- batched instances (include/quasar_mhd_batch.h) ------------------------
 int qmhd_batch_create(const qmhd_config* configs, int n, qmhd_batch** out) {
   return guarded([&] {

@@ -127,24 +127,77 @@ __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, 
 __device__ __forceinline__ double sq3(double x, double y, double z) {
   return add(add(mul(x, x), mul(y, y)), mul(z, z));
 }
+// Divisions of the functions below, all by a few divisors with several
+// numerators each.  PlainDiv: the division operator.
+struct PlainDiv {
+  struct By {
+    double b;
+    __device__ __forceinline__ double of(double a) const { return __ddiv_rn(a, b); }
+  };
+  __device__ __forceinline__ By by(double b) { return By{b}; }
+};
+// SharedDiv: the same bits from one correctly rounded reciprocal y per divisor
+// (two corrections of rcp_nr's operand by its residual; Markstein,
+// "Computation of Elementary Functions on the IBM RISC System/6000
+// Processor", 1990) and four FP64 instructions a quotient: q0 = RN(a yl + RN(a
+// y)), yl the remainder of y, is within an ulp of a / b, its residual a - b q0
+// is exact, and RN(q0 + (a - b q0) y) is then the correctly rounded quotient
+// (theorem 7.1 there).  A divisor outside 2^-900 .. 2^900 sets `bad`: the
+// caller repeats the work with PlainDiv.  A numerator below 1e-291 may come
+// out an ulp off, in sums that hold a term of order one.
+struct SharedDiv {
+  bool bad = false;
+  struct By {
+    double b, y, yl;
+    __device__ __forceinline__ double of(double a) const {
+      const double q = fma(a, yl, __dmul_rn(a, y));
+      return fma(fma(-b, q, a), y, q);
+    }
+  };
+  __device__ __forceinline__ By by(double b) {
+    bad = bad || ((unsigned(__double2hiint(b)) >> 20) & 0x7ffu) - 123u >= 1800u;
+    const double y0 = rcp_nr(b);
+    const double y = fma(y0, fma(-b, y0, 1.0), y0);
+    return By{b, y, fma(-b, y, 1.0) * y};
+  }
+};
+
 // mhd_state.hpp:92-100
-__device__ __forceinline__ double scaled_norm3(double x, double y, double z) {
+template <class D>
+__device__ __forceinline__ double scaled_norm3(D& dv, double x, double y, double z) {
   const double s = fmax(fabs(x), fmax(fabs(y), fabs(z)));
   if (s == 0.0) return 0.0;
-  return mul(s, sqrt(sq3(x / s, y / s, z / s)));
+  const auto q = dv.by(s);
+  return mul(s, sqrt(sq3(q.of(x), q.of(y), q.of(z))));
 }
 // mhd_state.hpp:105-114
-__device__ __forceinline__ double half_sq3(double x, double y, double z) {
+template <class D>
+__device__ __forceinline__ double half_sq3(D& dv, double x, double y, double z) {
   const double s = fmax(fabs(x), fmax(fabs(y), fabs(z)));
   if (s == 0.0) return 0.0;
-  return mul(mul(0.5, s), mul(s, sq3(x / s, y / s, z / s)));
+  const auto q = dv.by(s);
+  return mul(mul(0.5, s), mul(s, sq3(q.of(x), q.of(y), q.of(z))));
 }
-// mhd_state.hpp:118-128
-__device__ __forceinline__ double kin_mom(double mx, double my, double mz, double rho) {
+// mhd_state.hpp:118-128, with the quotient by sqrt(rho)
+template <class D, class Q>
+__device__ __forceinline__ double kin_mom(D& dv, double mx, double my, double mz, const Q& sr) {
   const double s = fmax(fabs(mx), fmax(fabs(my), fabs(mz)));
   if (s == 0.0) return 0.0;
-  const double q = s / sqrt(rho);
-  return mul(mul(0.5, q), mul(q, sq3(mx / s, my / s, mz / s)));
+  const auto d = dv.by(s);
+  const double q = sr.of(s);
+  return mul(mul(0.5, q), mul(q, sq3(d.of(mx), d.of(my), d.of(mz))));
+}
+__device__ __forceinline__ double scaled_norm3(double x, double y, double z) {
+  PlainDiv d;
+  return scaled_norm3(d, x, y, z);
+}
+__device__ __forceinline__ double half_sq3(double x, double y, double z) {
+  PlainDiv d;
+  return half_sq3(d, x, y, z);
+}
+__device__ __forceinline__ double kin_mom(double mx, double my, double mz, double rho) {
+  PlainDiv d;
+  return kin_mom(d, mx, my, mz, d.by(sqrt(rho)));
 }
 // mhd_state.hpp:131-141
 __device__ __forceinline__ double kin_vel(double rho, double vx, double vy, double vz) {
@@ -154,14 +207,14 @@ __device__ __forceinline__ double kin_vel(double rho, double vx, double vy, doub
   return mul(mul(0.5, q), mul(q, sq3(vx / s, vy / s, vz / s)));
 }
 // mhd_state.hpp:148-182, normal Alfven component along x
-__device__ __forceinline__ void magnetosonic(double rho, double p, double bn, double bt1,
+template <class D, class Q>
+__device__ __forceinline__ void magnetosonic(D& dv, const Q& sr, double p, double bn, double bt1,
                                              double bt2, double gamma, double& fast,
                                              double& slow, double& sound, double& can,
                                              double& ca) {
-  const double sr = sqrt(rho);
-  sound = (p > 0.0 && gamma > 0.0) ? mul(sqrt(gamma), sqrt(p) / sr) : 0.0;
-  const double ax = bn / sr, ay = bt1 / sr, az = bt2 / sr;
-  ca = scaled_norm3(ax, ay, az);
+  sound = (p > 0.0 && gamma > 0.0) ? mul(sqrt(gamma), sr.of(sqrt(p))) : 0.0;
+  const double ax = sr.of(bn), ay = sr.of(bt1), az = sr.of(bt2);
+  ca = scaled_norm3(dv, ax, ay, az);
   can = fabs(ax);
   const double scale = fmax(sound, ca);
   if (!(scale > 0.0)) {
@@ -169,7 +222,8 @@ __device__ __forceinline__ void magnetosonic(double rho, double p, double bn, do
     slow = 0.0;
     return;
   }
-  const double an = sound / scale, bnn = ca / scale, cn = can / scale;
+  const auto ds = dv.by(scale);
+  const double an = ds.of(sound), bnn = ds.of(ca), cn = ds.of(can);
   const double a2 = mul(an, an), b2 = mul(bnn, bnn), c2 = mul(cn, cn);
   const double sum = add(a2, b2);
   double disc = sub(mul(sum, sum), mul(mul(4.0, a2), c2));
@@ -180,10 +234,15 @@ __device__ __forceinline__ void magnetosonic(double rho, double p, double bn, do
   slow = mul(scale, sqrt(s2));
 }
 // mhd_state.hpp:185-191
-__device__ __forceinline__ double pressure(const St& u, double gamma) {
-  const double k = kin_mom(u.mx, u.my, u.mz, u.rho);
-  const double m = half_sq3(u.bx, u.by, u.bz);
+template <class D, class Q>
+__device__ __forceinline__ double pressure(D& dv, const Q& sr, const St& u, double gamma) {
+  const double k = kin_mom(dv, u.mx, u.my, u.mz, sr);
+  const double m = half_sq3(dv, u.bx, u.by, u.bz);
   return mul(sub(gamma, 1.0), sub(sub(u.E, k), m));
+}
+__device__ __forceinline__ double pressure(const St& u, double gamma) {
+  PlainDiv d;
+  return pressure(d, d.by(sqrt(u.rho)), u, gamma);
 }
 // Plain-arithmetic EOS for the places whose result depends continuously on
 // rounding (Riemann solver, CFL speeds, admissibility tests): one reciprocal
@@ -220,13 +279,6 @@ __device__ __forceinline__ St to_cons(const Pr& w, double igm) {
                 0.5 * (w.bx * w.bx + w.by * w.by + w.bz * w.bz),
             w.bx, w.by, w.bz};
 }
-// mhd_state.hpp:272-289 (x-normal)
-__device__ __forceinline__ double fast_x(const St& u, double gamma) {
-  double f, s, a, cn, ca;
-  magnetosonic(u.rho, pressure(u, gamma), u.bx, u.by, u.bz, gamma, f, s, a, cn, ca);
-  return f;
-}
-
 // x<->y swap of the in-plane momentum and field (mhd_reconstruct.hip:167-176,
 // hlld_core.hpp:45-61).
 __device__ __forceinline__ St swap_xy(const St& v) {

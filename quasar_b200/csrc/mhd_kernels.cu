@@ -408,28 +408,31 @@ constexpr double kRs2 = 0.7071067811865475;  // 1/sqrt(2) rounded
 // entries (velocities, transverse unit vector, 1/a^2, |v|^2/2) share one
 // reciprocal each instead of a division per term (a rounding-level
 // difference).
-__device__ __forceinline__ Eg eig_scalars(const St& s, double gamma) {
+template <class D>
+__device__ __forceinline__ Eg eig_scalars_by(D& dv, const St& s, double gamma) {
   Eg e;
-  const double ir = 1.0 / s.rho;
-  const Pr w{s.rho, s.mx * ir, s.my * ir, s.mz * ir, pressure(s, gamma), s.bx, s.by, s.bz};
-  e.rho = w.rho;
-  const double p = w.p > 0.0 ? w.p : 0.0;
+  e.rho = s.rho;
   e.sr = sqrt(e.rho);
+  const auto dsr = dv.by(e.sr);
+  const double ir = 1.0 / s.rho;
+  const Pr w{s.rho, s.mx * ir, s.my * ir, s.mz * ir, pressure(dv, dsr, s, gamma), s.bx, s.by, s.bz};
+  const double p = w.p > 0.0 ? w.p : 0.0;
   e.bt1 = w.by;
   e.bt2 = w.bz;
   double cax, ca, den, clip = 0.0;
-  magnetosonic(e.rho, p, w.bx, w.by, w.bz, gamma, e.cf, e.cs, e.a, cax, ca);
+  magnetosonic(dv, dsr, p, w.bx, w.by, w.bz, gamma, e.cf, e.cs, e.a, cax, ca);
   {
-    const double sc = e.cf > 0.0 ? e.cf : 1.0;
-    const double cfn = e.cf / sc, csn = e.cs / sc, an = e.a / sc;
+    const auto sc = dv.by(e.cf > 0.0 ? e.cf : 1.0);
+    const double cfn = sc.of(e.cf), csn = sc.of(e.cs), an = sc.of(e.a);
     den = sub(mul(cfn, cfn), mul(csn, csn));
     if (den <= mul(64.0 * kEps, add(mul(cfn, cfn), mul(csn, csn)))) {
       e.af = kRs2;
       e.as = kRs2;
       den = 0.0;
     } else {
-      const double af2 = sub(mul(an, an), mul(csn, csn)) / den;
-      const double as2 = sub(mul(cfn, cfn), mul(an, an)) / den;
+      const auto dd = dv.by(den);
+      const double af2 = dd.of(sub(mul(an, an), mul(csn, csn)));
+      const double as2 = dd.of(sub(mul(cfn, cfn), mul(an, an)));
       e.af = sqrt(af2 < 0.0 ? 0.0 : af2);
       e.as = sqrt(as2 < 0.0 ? 0.0 : as2);
       const double least = af2 < as2 ? af2 : as2;
@@ -437,9 +440,9 @@ __device__ __forceinline__ Eg eig_scalars(const St& s, double gamma) {
     }
   }
   {
-    const double bt = scaled_norm3(w.by, w.bz, 0.0);
+    const double bt = scaled_norm3(dv, w.by, w.bz, 0.0);
     const double fs = e.a > ca ? e.a : ca;
-    if (bt == 0.0 || bt / e.sr <= 64.0 * kEps * (fs + kTiny)) {
+    if (bt == 0.0 || dsr.of(bt) <= 64.0 * kEps * (fs + kTiny)) {
       e.b1 = kRs2;
       e.b2 = kRs2;
     } else {
@@ -486,6 +489,22 @@ __device__ __forceinline__ Eg eig_scalars(const St& s, double gamma) {
     e.sure = (80.0 - W * F) * den >= k * k * fma(den * clip, 3.8e14, 1.0);
   }
   return e;
+}
+
+__device__ __noinline__ Eg eig_scalars_plain(const St& s, double gamma) {
+  PlainDiv d;
+  return eig_scalars_by(d, s, gamma);
+}
+// The eigen scalars are a quarter of the reconstruction's instructions and one
+// long dependent chain, most of it 26 divisions by twelve divisors; sharing
+// each divisor's reciprocal keeps the bits (flow 2048^2 MP7 reconstruction
+// 6.29 -> 5.86 ms per step, rotor 4096^2 26.0 -> 23.0).  Divisors outside the
+// shared form's range are tested once at the end: a select per quotient
+// measured slower than the divisions.
+__device__ __forceinline__ Eg eig_scalars(const St& s, double gamma) {
+  SharedDiv d;
+  const Eg e = eig_scalars_by(d, s, gamma);
+  return d.bad ? eig_scalars_plain(s, gamma) : e;
 }
 
 // Primitive left row and right column of wave k (mhd_eigensystem.hpp:176-320);
@@ -3355,6 +3374,18 @@ __global__ void k_probe_roots(const double* __restrict__ x, long long n, double*
   if (k >= n) return;
   y[k] = rcp_nr(x[k]);
   z[k] = rsqrt_nr(x[k]);
+}
+__global__ void k_probe_quotients(const double* __restrict__ a, const double* __restrict__ b,
+                                  long long n, double* q) {
+  const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  SharedDiv d;
+  const double v = d.by(b[k]).of(a[k]);
+  q[k] = d.bad ? __ddiv_rn(a[k], b[k]) : v;
+}
+void launch_probe_quotients(const double* a, const double* b, long long n, double* q,
+                            cudaStream_t s) {
+  if (n > 0) k_probe_quotients<<<cdiv(n, 256), 256, 0, s>>>(a, b, n, q);
 }
 void launch_probe_roots(const double* x, long long n, double* y, double* z, cudaStream_t s) {
   if (n > 0) k_probe_roots<<<cdiv(n, 256), 256, 0, s>>>(x, n, y, z);

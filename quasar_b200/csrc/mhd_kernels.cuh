@@ -312,6 +312,9 @@ void launch_face_lists(const Grid& g, const unsigned char* flag, int* xlist, int
 
 // y[k] and z[k] = the stage kernels' reciprocal and inverse square root of x[k].
 void launch_probe_roots(const double* x, long long n, double* y, double* z, cudaStream_t s);
+// q[k] = a[k] / b[k] as the eigen scalars divide.
+void launch_probe_quotients(const double* a, const double* b, long long n, double* q,
+                            cudaStream_t s);
 
 // *bad |= 1 if any of v[0..n) is not finite (*bad must start at zero).
 void launch_flag_nonfinite(const double* v, long long n, unsigned long long* bad, cudaStream_t s);
