@@ -1278,10 +1278,18 @@ __device__ __forceinline__ void b_reconstruct(const Grid& g, const StateP& u, co
   recon_face<DIR, ORDER, MODE>(g, u, out, gamma, i, j, label, defer);
 }
 
-template <int DIR, int ORDER>
-__global__ void __launch_bounds__(128, 4) k_reconstruct(Grid g, StateP u, IfaceP out, double gamma,
-                                                        const Ctl* ctl) {
-  b_reconstruct<DIR, ORDER>(g, u, out, gamma, ctl, blockIdx.x, blockIdx.y);
+// The faces of one direction (dir0 + blockIdx.z) or, with two layers of
+// blocks, of both in one launch: the y faces' blocks fill the SMs while the x
+// faces' last ones drain, and a grid that does not fill the chip (a 64^2 grid
+// has 37 blocks a direction) runs both side by side.  64^2 MP5 step 0.26 ->
+// 0.18 ms with the face flux launched the same way.
+template <int ORDER>
+__global__ void __launch_bounds__(128, 4) k_reconstruct(Grid g, StateP u, IfaceP ix, IfaceP iy,
+                                                        double gamma, const Ctl* ctl, int dir0) {
+  if (dir0 + int(blockIdx.z) == 0)
+    b_reconstruct<0, ORDER>(g, u, ix, gamma, ctl, blockIdx.x, blockIdx.y);
+  else
+    b_reconstruct<1, ORDER>(g, u, iy, gamma, ctl, blockIdx.x, blockIdx.y);
 }
 
 // Limiter labels of the cells (training data of the indicator): the
@@ -1696,16 +1704,16 @@ __device__ __forceinline__ Fx flat_flux(const St& s, double p, double ir) {
 template <int DIR, int ORDER, int TX = kFqTX>
 __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, const FluxP& out,
                                                double* emf, int* nj, double* spd, double gamma,
-                                               const Ctl* ctl, int bx, int by) {
+                                               const Ctl* ctl, int bx, int by, double* sm) {
   constexpr int H = ORDER == 5 ? 2 : 3, N = 2 * H + 1, Q = ORDER == 5 ? 3 : 4;
   constexpr int FPW = 32 / Q, TY = fq_ty<ORDER>();         // faces per warp, tile rows
   static_assert(4 * FPW == TX * TY, "four warps cover the face tile");
   constexpr int TR = DIR == 0 ? TY + 2 * H : TY;          // tile rows (j)
   constexpr int TC = DIR == 0 ? TX : TX + 2 * H;          // tile columns (i)
-  __shared__ double tile[16][TR][TC];
+  double(*tile)[TR][TC] = reinterpret_cast<double(*)[TR][TC]>(sm);
   // staged and L == R in every component: one bit per tile slot
   constexpr int kWords = (TR * TC + 31) / 32;
-  __shared__ unsigned same[kWords + 1];
+  unsigned* same = reinterpret_cast<unsigned*>(sm + 16 * TR * TC);
   if (ctl->status) return;  // uniform over the block
   const int i0 = bx * TX, j0 = by * TY;
   const bool perx = g.bc[0] == 0 && g.bc[1] == 0, pery = g.bc[2] == 0 && g.bc[3] == 0;
@@ -1873,21 +1881,34 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
 }
 
 // Component-split recovery (MP7), as described above.
-template <int DIR, int ORDER, int TX = kFqTX>
+// sm: the caller's shared memory (fq_smem doubles), or null (OWN) where the
+// kernel holds only this body and has arrays of its own.
+template <int DIR, int ORDER, bool OWN, int TX = kFqTX>
 __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, const FluxP& out,
                                                double* emf, int* nj, double* spd, double gamma,
-                                               const Ctl* ctl, int bx, int by) {
+                                               const Ctl* ctl, int bx, int by, double* sm) {
   constexpr int H = ORDER == 5 ? 2 : 3, N = 2 * H + 1, Q = ORDER == 5 ? 3 : 4;
   constexpr int FPW = 32 / Q, TY = fq_ty<ORDER>();         // faces per warp, tile rows
   static_assert(4 * FPW == TX * TY, "four warps cover the face tile");
   constexpr int TR = DIR == 0 ? TY + 2 * H : TY;          // tile rows (j)
   constexpr int TC = DIR == 0 ? TX : TX + 2 * H;          // tile columns (i)
   constexpr int PS = fq_plane(TR * TC), FS = fq_face<ORDER>();
-  __shared__ double tile[16 * PS];             // component c of slot (row, col): c PS + row TC + col
-  // staged and L == R in every component: one bit per tile slot
   constexpr int kWords = (TR * TC + 31) / 32;
-  __shared__ unsigned same[kWords + 1];
-  __shared__ __align__(16) double pts[4 * FPW * FS];  // per face: Q point rows
+  double* tile;    // component c of slot (row, col): c PS + row TC + col
+  unsigned* same;  // staged and L == R in every component: one bit per tile slot
+  double* pts;     // per face: Q point rows
+  if constexpr (OWN) {
+    __shared__ double own_tile[16 * PS];
+    __shared__ unsigned own_same[kWords + 1];
+    __shared__ __align__(16) double own_pts[4 * FPW * FS];
+    tile = own_tile;
+    same = own_same;
+    pts = own_pts;
+  } else {
+    tile = sm;
+    pts = sm + 16 * PS;
+    same = reinterpret_cast<unsigned*>(pts + 4 * FPW * FS);
+  }
   if (ctl->status) return;  // uniform over the block
   const int i0 = bx * TX, j0 = by * TY;
   const bool perx = g.bc[0] == 0 && g.bc[1] == 0, pery = g.bc[2] == 0 && g.bc[3] == 0;
@@ -2074,23 +2095,62 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
   if (lane == 0) nj[k] = nproof == 0 ? 1 : 0;
 }
 
+// Shared memory (doubles) of one direction's tile, point rows and bits.
+template <int DIR, int ORDER>
+constexpr int fq_smem() {
+  constexpr int H = ORDER == 5 ? 2 : 3, TY = fq_ty<ORDER>();
+  constexpr int cells = DIR == 0 ? (TY + 2 * H) * kFqTX : TY * (kFqTX + 2 * H), bits = 4;
+  if (ORDER == 5) return 16 * cells + bits;
+  return 16 * fq_plane(cells) + 32 * fq_face<ORDER>() + bits;
+}
+template <int ORDER>
+constexpr int fq_smem_both() {
+  return fq_smem<0, ORDER>() > fq_smem<1, ORDER>() ? fq_smem<0, ORDER>() : fq_smem<1, ORDER>();
+}
 // TX: faces per tile row; the block is four warps of 32 / Q groups each.
-template <int DIR, int ORDER, int TX = kFqTX>
+template <int DIR, int ORDER, bool OWN, int TX = kFqTX>
 __device__ __forceinline__ void b_face_flux_qs(const Grid& g, const IfaceP& in, const FluxP& out,
                                                double* emf, int* nj, double* spd, double gamma,
-                                               const Ctl* ctl, int bx, int by) {
+                                               const Ctl* ctl, int bx, int by, double* sm) {
   if constexpr (ORDER == 7)
-    b_face_flux_cs<DIR, ORDER, TX>(g, in, out, emf, nj, spd, gamma, ctl, bx, by);
+    b_face_flux_cs<DIR, ORDER, OWN, TX>(g, in, out, emf, nj, spd, gamma, ctl, bx, by, sm);
   else
-    b_face_flux_pt<DIR, ORDER, TX>(g, in, out, emf, nj, spd, gamma, ctl, bx, by);
+    b_face_flux_pt<DIR, ORDER, TX>(g, in, out, emf, nj, spd, gamma, ctl, bx, by, sm);
 }
 
+// Outputs of one direction's face flux.
+struct FaceOut {
+  FluxP f;
+  double* emf;
+  int* nj;
+  double* spd;
+};
+// One direction per launch, for MP7 grids beyond kFqPairBlocks.
 template <int DIR, int ORDER>
 __global__ void __launch_bounds__(kFqThreads, kFqBlocksPerSm)
-    k_face_flux_qs(Grid g, IfaceP in, FluxP out, double* emf, int* nj, double* spd, double gamma,
-                   const Ctl* ctl) {
-  b_face_flux_qs<DIR, ORDER, kFqTX>(g, in, out, emf, nj, spd, gamma, ctl, blockIdx.x,
-                                          blockIdx.y);
+    k_face_flux_one(Grid g, IfaceP in, FluxP out, double* emf, int* nj, double* spd, double gamma,
+                    const Ctl* ctl) {
+  b_face_flux_qs<DIR, ORDER, true, kFqTX>(g, in, out, emf, nj, spd, gamma, ctl, blockIdx.x,
+                                          blockIdx.y, nullptr);
+}
+// One direction (dir0 + blockIdx.z) or both, as k_reconstruct.  At MP5 the
+// pair is faster at every size (1024^2: 1.35 -> 1.32 ms per step).  At MP7 the
+// kernel that holds both bodies is slower where the grid fills the chip many
+// times over (1024^2: 1.38 -> 1.51) and faster where it does not (64^2: 0.060 ->
+// 0.042, 200 x 150, 988 blocks a direction: 0.086 -> 0.075): the line is two
+// waves of resident blocks.
+constexpr long long kFqPairBlocks = 2 * 148 * kFqBlocksPerSm;
+template <int ORDER>
+__global__ void __launch_bounds__(kFqThreads, kFqBlocksPerSm)
+    k_face_flux_qs(Grid g, IfaceP ix, IfaceP iy, FaceOut ox, FaceOut oy, double gamma,
+                   const Ctl* ctl, int dir0) {
+  __shared__ __align__(16) double sm[fq_smem_both<ORDER>()];
+  if (dir0 + int(blockIdx.z) == 0)
+    b_face_flux_qs<0, ORDER, false, kFqTX>(g, ix, ox.f, ox.emf, ox.nj, ox.spd, gamma, ctl, blockIdx.x,
+                                    blockIdx.y, sm);
+  else
+    b_face_flux_qs<1, ORDER, false, kFqTX>(g, iy, oy.f, oy.emf, oy.nj, oy.spd, gamma, ctl, blockIdx.x,
+                                    blockIdx.y, sm);
 }
 
 }  // namespace
@@ -3001,14 +3061,15 @@ __global__ void kb_face_lists(const BatchRec* __restrict__ r, const BatchLearnRe
 template <int DIR, int ORDER>
 __global__ void __launch_bounds__(kFqThreads, kFqBlocksPerSm)
     kb_face_flux_q(const BatchRec* __restrict__ r, BatchPlan p, int speeds) {
+  __shared__ __align__(16) double sm[ORDER == 5 ? fq_smem<DIR, 5>() : 2];
   for (int t = blockIdx.x; t < p.total; t += gridDim.x) {
     int local, bx, by;
     const BatchRec& q = r[batch_locate(p, t, &local)];
     batch_block(kBpFlux, q.a.g, local, &bx, &by);
-    b_face_flux_qs<DIR, ORDER, kFqTX>(q.a.g, DIR == 0 ? q.a.ix : q.a.iy, DIR == 0 ? q.a.fx : q.a.fy,
+    b_face_flux_qs<DIR, ORDER, ORDER == 7, kFqTX>(q.a.g, DIR == 0 ? q.a.ix : q.a.iy, DIR == 0 ? q.a.fx : q.a.fy,
                                DIR == 0 ? q.a.xemf : q.a.yemf, DIR == 0 ? q.a.xnj : q.a.ynj,
                                speeds ? (DIR == 0 ? q.a.xspd : q.a.yspd) : nullptr, q.a.gamma,
-                               q.a.ctl, bx, by);
+                               q.a.ctl, bx, by, sm);
     __syncthreads();  // the shared tile is reused by the next tile
   }
 }
@@ -3131,55 +3192,76 @@ void launch_colloc_check(const Grid& g, const StateP& cand, const StateP* base, 
   }
 }
 
-template <int DIR, int ORDER>
-static void recon_launch(const StageArgs& a, cudaStream_t s) {
+// dir 0 or 1: that direction's faces; 2: both.
+template <int ORDER>
+static void recon_launch(const StageArgs& a, int dir, cudaStream_t s) {
   const Grid& g = a.g;
-
   const dim3 block(kBX, 4);
-  const int ni = DIR == 0 ? g.nx + 1 : g.nx + 2 * g.ng;
-  const int nj = DIR == 0 ? g.ny + 2 * g.ng : g.ny + 1;
-  const dim3 grid(cdiv(ni, kBX), cdiv(nj, 4));
+  const int ni = dir == 0 ? g.nx + 1 : g.nx + 2 * g.ng;
+  const int nj = dir == 1 ? g.ny + 1 : g.ny + 2 * g.ng;
+  const dim3 grid(cdiv(ni, kBX), cdiv(nj, 4), dir == 2 ? 2 : 1);
   size_t smem = 0;
   if (ORDER == 5 || ORDER == 7) {
     smem = kReconWarpSmem;
-    ensure_smem((const void*)k_reconstruct<DIR, ORDER>, smem);
+    ensure_smem((const void*)k_reconstruct<ORDER>, smem);
   }
-  k_reconstruct<DIR, ORDER><<<grid, block, smem, s>>>(g, a.u, DIR == 0 ? a.ix : a.iy, a.gamma,
-                                                      a.ctl);
+  k_reconstruct<ORDER><<<grid, block, smem, s>>>(g, a.u, a.ix, a.iy, a.gamma, a.ctl,
+                                                 dir == 1 ? 1 : 0);
 }
 
 void launch_reconstruct(const StageArgs& a, int dir, cudaStream_t s) {
-#define QB_RECON(D, O) \
-  if (dir == D && a.order == O) return recon_launch<D, O>(a, s);
-  QB_RECON(0, 1) QB_RECON(1, 1) QB_RECON(0, 2) QB_RECON(1, 2)
-  QB_RECON(0, 5) QB_RECON(1, 5) QB_RECON(0, 7) QB_RECON(1, 7)
-#undef QB_RECON
+  switch (a.order) {
+    case 1: return recon_launch<1>(a, dir, s);
+    case 2: return recon_launch<2>(a, dir, s);
+    case 5: return recon_launch<5>(a, dir, s);
+    default: return recon_launch<7>(a, dir, s);
+  }
 }
 
 template <int DIR, int ORDER>
-static void flux_launch(const StageArgs& a, bool speeds, cudaStream_t s) {
+static void flux_low_launch(const StageArgs& a, bool speeds, cudaStream_t s) {
   const Grid& g = a.g;
-  if (ORDER == 5 || ORDER == 7) {
-    constexpr int O = ORDER == 5 ? 5 : 7;
-    const dim3 grid(cdiv(g.nx + 1, kFqTX), cdiv(g.ny + 1, fq_ty<O>()));
-    k_face_flux_qs<DIR, O><<<grid, kFqThreads, 0, s>>>(
-        g, DIR == 0 ? a.ix : a.iy, DIR == 0 ? a.fx : a.fy, DIR == 0 ? a.xemf : a.yemf,
-        DIR == 0 ? a.xnj : a.ynj, speeds ? (DIR == 0 ? a.xspd : a.yspd) : nullptr, a.gamma, a.ctl);
-    return;
-  }
   const dim3 block(kBX, 4);
   const dim3 grid(cdiv(g.nx + 1, kBX), cdiv(g.ny + 1, 4));
   k_face_flux<DIR, ORDER><<<grid, block, 0, s>>>(
       g, DIR == 0 ? a.ix : a.iy, DIR == 0 ? a.fx : a.fy, DIR == 0 ? a.xemf : a.yemf,
       DIR == 0 ? a.xnj : a.ynj, speeds ? (DIR == 0 ? a.xspd : a.yspd) : nullptr, a.gamma, a.ctl);
 }
+template <int ORDER>
+static void flux_launch(const StageArgs& a, int dir, bool speeds, cudaStream_t s) {
+  const Grid& g = a.g;
+  const dim3 grid(cdiv(g.nx + 1, kFqTX), cdiv(g.ny + 1, fq_ty<ORDER>()), dir == 2 ? 2 : 1);
+  const FaceOut ox{a.fx, a.xemf, a.xnj, speeds ? a.xspd : nullptr};
+  const FaceOut oy{a.fy, a.yemf, a.ynj, speeds ? a.yspd : nullptr};
+  if constexpr (ORDER == 7) {
+    if ((long long)grid.x * grid.y > kFqPairBlocks) {
+      const dim3 one(grid.x, grid.y);
+      if (dir != 1)
+        k_face_flux_one<0, ORDER><<<one, kFqThreads, 0, s>>>(g, a.ix, a.fx, a.xemf, a.xnj, ox.spd,
+                                                             a.gamma, a.ctl);
+      if (dir != 0)
+        k_face_flux_one<1, ORDER><<<one, kFqThreads, 0, s>>>(g, a.iy, a.fy, a.yemf, a.ynj, oy.spd,
+                                                             a.gamma, a.ctl);
+      return;
+    }
+  }
+  k_face_flux_qs<ORDER><<<grid, kFqThreads, 0, s>>>(g, a.ix, a.iy, ox, oy, a.gamma, a.ctl,
+                                                    dir == 1 ? 1 : 0);
+}
 
 void launch_face_flux(const StageArgs& a, int dir, bool speeds, cudaStream_t s) {
-#define QB_FLUX(D, O) \
-  if (dir == D && a.order == O) return flux_launch<D, O>(a, speeds, s);
-  QB_FLUX(0, 1) QB_FLUX(1, 1) QB_FLUX(0, 2) QB_FLUX(1, 2)
-  QB_FLUX(0, 5) QB_FLUX(1, 5) QB_FLUX(0, 7) QB_FLUX(1, 7)
-#undef QB_FLUX
+  switch (a.order) {
+    case 1:
+      if (dir != 1) flux_low_launch<0, 1>(a, speeds, s);
+      if (dir != 0) flux_low_launch<1, 1>(a, speeds, s);
+      break;
+    case 2:
+      if (dir != 1) flux_low_launch<0, 2>(a, speeds, s);
+      if (dir != 0) flux_low_launch<1, 2>(a, speeds, s);
+      break;
+    case 5: return flux_launch<5>(a, dir, speeds, s);
+    default: return flux_launch<7>(a, dir, speeds, s);
+  }
 }
 
 template <int ORDER>

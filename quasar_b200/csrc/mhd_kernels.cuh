@@ -113,6 +113,7 @@ void launch_fill_ghosts(const Grid& g, const StateP& u, cudaStream_t s);
 void launch_colloc_check(const Grid& g, const StateP& cand, const StateP* base,
                          int theta_mask, bool anchor_check, bool live_checks,
                          bool solver_owned, double gamma, Ctl* ctl, cudaStream_t s);
+// dir: 0 the x faces, 1 the y faces, 2 both.
 void launch_reconstruct(const StageArgs& a, int dir, cudaStream_t s);
 void launch_face_flux(const StageArgs& a, int dir, bool speeds, cudaStream_t s);
 void launch_cell_emf(const StageArgs& a, bool cfl_reduce, cudaStream_t s);

@@ -345,8 +345,7 @@ void MhdSolver2D::front_impl(int order, int dt_mode, int anchor_mode) {
   reconstruct_stage(a, order);
   mark(1);
   const bool speeds = dt_mode != 0;
-  launch_face_flux(a, 0, speeds, stream_);
-  launch_face_flux(a, 1, speeds, stream_);
+  launch_face_flux(a, 2, speeds, stream_);
   mark(2);
   launch_cell_emf(a, speeds, stream_);
   mark(3);
@@ -368,8 +367,7 @@ void MhdSolver2D::reconstruct_stage(const StageArgs& a, int order) {
     launch_reconstruct_learned(a, 0, flags_, flists_, fcounts_, 4 * sms, stream_);
     launch_reconstruct_learned(a, 1, flags_, flists_ + g_.size(), fcounts_ + 1, 4 * sms, stream_);
   } else {
-    launch_reconstruct(a, 0, stream_);
-    launch_reconstruct(a, 1, stream_);
+    launch_reconstruct(a, 2, stream_);
   }
 }
 
@@ -436,8 +434,7 @@ void MhdSolver2D::finish_impl(int order, const double* dt_dev, double dt_host, b
     const StageArgs a = stage_args(in, order);
     reconstruct_stage(a, order);
     mark(1);
-    launch_face_flux(a, 0, false, stream_);
-    launch_face_flux(a, 1, false, stream_);
+    launch_face_flux(a, 2, false, stream_);
     mark(2);
     launch_cell_emf(a, false, stream_);
     mark(3);
