@@ -2406,16 +2406,10 @@ __device__ __forceinline__ void b_cell_emf_s(const Grid& g, const StateP& u, dou
         double smp[N];
 #pragma unroll
         for (int t = 0; t < N; ++t) smp[t] = X[(c * SY + threadIdx.y + t) * TX + threadIdx.x];
-        if constexpr (ORDER == 7) {
-          // the constant-stencil test once for the four y-nodes
-          double pv[Q];
-          point_values<ORDER>(smp, pv);
+        double pv[Q];
+        point_values<ORDER>(smp, pv);
 #pragma unroll
-          for (int qy = 0; qy < Q; ++qy) st[qy][c] = pv[qy];
-        } else {
-#pragma unroll
-          for (int qy = 0; qy < Q; ++qy) st[qy][c] = point_value<ORDER>(qy, smp);
-        }
+        for (int qy = 0; qy < Q; ++qy) st[qy][c] = pv[qy];
       }
 #pragma unroll
       for (int qy = 0; qy < Q; ++qy) {
@@ -4069,9 +4063,6 @@ __device__ double abi_face_rate(const Grid& g, const IfaceP& in, int i, int j, d
   constexpr int H = ORDER == 5 ? 2 : 3, N = 2 * H + 1, Q = ORDER == 5 ? 3 : 4;
   const long long ts = DIR == 0 ? g.pitch : 1;
   for (int q = 0; q < Q; ++q) {
-    double w[N];
-#pragma unroll
-    for (int t = 0; t < N; ++t) w[t] = point_w<ORDER>(q, t);
     double pl[8], pr[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -4081,8 +4072,17 @@ __device__ double abi_face_rate(const Grid& g, const IfaceP& in, int i, int j, d
         sa[t] = in.L[c][ks + (t - H) * ts];
         sb[t] = in.R[c][ks + (t - H) * ts];
       }
-      pl[c] = wsum<N>(w, sa);
-      pr[c] = wsum<N>(w, sb);
+      // the face flux's own sums: all nodes at once at MP7, one at MP5
+      if (ORDER == 7) {
+        double va[Q], vb[Q];
+        point_values<ORDER>(sa, va);
+        point_values<ORDER>(sb, vb);
+        pl[c] = q == 0 ? va[0] : q == 1 ? va[1] : q == 2 ? va[2] : va[Q - 1];
+        pr[c] = q == 0 ? vb[0] : q == 1 ? vb[1] : q == 2 ? vb[2] : vb[Q - 1];
+      } else {
+        pl[c] = point_value<ORDER>(q, sa);
+        pr[c] = point_value<ORDER>(q, sb);
+      }
     }
     const St l{pl[0], pl[1], pl[2], pl[3], pl[4], pl[5], pl[6], pl[7]};
     const St r{pr[0], pr[1], pr[2], pr[3], pr[4], pr[5], pr[6], pr[7]};
