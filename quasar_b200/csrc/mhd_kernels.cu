@@ -861,9 +861,21 @@ __device__ __forceinline__ void wave_pair(const Eg& e, int r, WavePair& w) {
   w.rt[6] = r6;
 }
 
+// The reconstructed components (rho, m_n, m_t1, m_t2, E, B_t1, B_t2) of a cell.
+template <int DIR>
+__device__ __forceinline__ void cell7(const StateP& u, long long k, double* v) {
+  v[0] = __ldg(u.c[0] + k);
+  v[1] = __ldg(u.c[DIR == 0 ? 1 : 2] + k);
+  v[2] = __ldg(u.c[DIR == 0 ? 2 : 1] + k);
+  v[3] = __ldg(u.c[3] + k);
+  v[4] = __ldg(u.c[4] + k);
+  v[5] = __ldg((DIR == 0 ? u.byc : u.bxc) + k);
+  v[6] = __ldg(u.c[7] + k);
+}
+
 // One warp's 32 faces (lane = face; `valid` false for lanes without one).
 // All lanes of the warp must call it; `ws` is the warp's shared memory.
-template <int DIR, int ORDER>
+template <int DIR, int ORDER, bool EARLY = false>
 __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out, double gamma,
                               int i, int j, bool valid, double* ws) {
   constexpr int H = ORDER == 5 ? 2 : 3;
@@ -916,8 +928,18 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
     const bool on = (vmask >> f) & 1u;
     const long long kf = __shfl_sync(0xffffffffu, k0, f);
     WavePair w;
-    bool ok = true;
+    // the stencil cells rl and rl + 4 (canonical frame; the normal field is not
+    // reconstructed).  EARLY: in flight while the wave vectors are formed
+    // (MP5 1024^2: 1.46 -> 1.40 ms per step).  At MP7 and in the batched and
+    // listed kernels that spills, and they are loaded where they are used
+    // (MP7 2048^2: 5.7 against 6.3 ms; batched MP5 1.02 against 1.09).
+    double ca[7], cb[7];
+    auto load_cells = [&] {
+      cell7<DIR>(u, kf + (long long)(rl - 1 - H) * step, ca);
+      if (rl + 4 < S) cell7<DIR>(u, kf + (long long)(rl + 3 - H) * step, cb);
+    };
     if (on) {
+      if (EARLY) load_cells();
       const double* r = rec + f;
       Eg e;
       e.rho = r[(kRecC + 0) * kRecS];
@@ -983,23 +1005,19 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
       const unsigned okm = __ballot_sync(0xffffffffu, ok);
       usable = ((okm >> (gi * 4)) & 0xFu) == 0xFu;
     }
-    // stencil deltas in the canonical frame: lane rl loads cells rl, rl + 4
+    // stencil deltas of this lane's cells
     if (on) {
+      if (!EARLY) load_cells();
       const double* r = rec + f;
+      const double c7[7] = {r[(kRecC + 0) * kRecS], r[(kRecC + 1) * kRecS], r[(kRecC + 2) * kRecS],
+                            r[(kRecC + 3) * kRecS], r[(kRecC + 4) * kRecS], r[(kRecC + 6) * kRecS],
+                            r[(kRecC + 7) * kRecS]};
+      double* dd = grp + kGrpD + rl * 7;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int sc = rl + 4 * h;
-        if (sc < S) {
-          const St d = rot<DIR>(load_cell(u, kf + (long long)(sc - 1 - H) * step));
-          double* dd = grp + kGrpD + sc * 7;
-          dd[0] = d.rho - r[(kRecC + 0) * kRecS];
-          dd[1] = d.mx - r[(kRecC + 1) * kRecS];
-          dd[2] = d.my - r[(kRecC + 2) * kRecS];
-          dd[3] = d.mz - r[(kRecC + 3) * kRecS];
-          dd[4] = d.E - r[(kRecC + 4) * kRecS];
-          dd[5] = d.by - r[(kRecC + 6) * kRecS];
-          dd[6] = d.bz - r[(kRecC + 7) * kRecS];
-        }
+      for (int v = 0; v < 7; ++v) dd[v] = ca[v] - c7[v];
+      if (rl + 4 < S) {
+#pragma unroll
+        for (int v = 0; v < 7; ++v) dd[28 + v] = cb[v] - c7[v];
       }
     }
     __syncwarp();
@@ -1258,7 +1276,7 @@ __device__ __forceinline__ void finish_face(const Grid& g, const StateP& u, cons
   }
 }
 
-template <int DIR, int ORDER, int MODE = 0>
+template <int DIR, int ORDER, int MODE = 0, bool EARLY = false>
 __device__ __forceinline__ void b_reconstruct(const Grid& g, const StateP& u, const IfaceP& out,
                                               double gamma, const Ctl* ctl, int bx, int by,
                                               int* label = nullptr,
@@ -1271,7 +1289,8 @@ __device__ __forceinline__ void b_reconstruct(const Grid& g, const StateP& u, co
   if constexpr (MODE == 0 && ORDER >= 5) {
     // the characteristic path, warp-cooperative (threadIdx.y = warp)
     extern __shared__ double dsm[];
-    mp_faces_warp<DIR, ORDER>(g, u, out, gamma, i, j, valid, dsm + threadIdx.y * kWarpReconDoubles);
+    mp_faces_warp<DIR, ORDER, EARLY>(g, u, out, gamma, i, j, valid,
+                                     dsm + threadIdx.y * kWarpReconDoubles);
     return;
   }
   if (!valid) return;
@@ -1287,9 +1306,9 @@ template <int ORDER>
 __global__ void __launch_bounds__(128, 4) k_reconstruct(Grid g, StateP u, IfaceP ix, IfaceP iy,
                                                         double gamma, const Ctl* ctl, int dir0) {
   if (dir0 + int(blockIdx.z) == 0)
-    b_reconstruct<0, ORDER>(g, u, ix, gamma, ctl, blockIdx.x, blockIdx.y);
+    b_reconstruct<0, ORDER, 0, ORDER == 5>(g, u, ix, gamma, ctl, blockIdx.x, blockIdx.y);
   else
-    b_reconstruct<1, ORDER>(g, u, iy, gamma, ctl, blockIdx.x, blockIdx.y);
+    b_reconstruct<1, ORDER, 0, ORDER == 5>(g, u, iy, gamma, ctl, blockIdx.x, blockIdx.y);
 }
 
 // Limiter labels of the cells (training data of the indicator): the
@@ -2598,6 +2617,7 @@ __device__ __forceinline__ void b_corner_emf_s(const Grid& g, const double* cell
   auto mapx = [&](int q) { return inner ? q : face_index(q, g.nx, g.bc[0], g.bc[1]); };
   auto mapy = [&](int q) { return inner ? q : face_index(q, g.ny, g.bc[2], g.bc[3]); };
   // column tx (and the NT - 1 beyond 32) of every row by the warp's row ty
+#pragma unroll
   for (int b = ty; b < TH; b += 8) {
     const int mj = mapy(j0 + LO + b);
     const long long row = g.idx(0, mj);
@@ -2607,6 +2627,7 @@ __device__ __forceinline__ void b_corner_emf_s(const Grid& g, const double* cell
     sxe[b][tx] = __ldg(xemf + row + fi);
     sxn[b][tx] = __ldg(xnj + row + fi) != 0;
   }
+#pragma unroll
   for (int b = ty; b < TY; b += 8) {
     const int fj = mapy(j0 + b);
     const long long row = g.idx(0, fj);
