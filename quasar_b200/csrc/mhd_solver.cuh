@@ -123,6 +123,7 @@ class MhdSolver2D {
   double cfl_limit_for(int coll);
   void check_cuda(const char* what);
   void build_graphs();
+  bool api_graphs();
 
   Config cfg_;
   Grid g_;
@@ -154,6 +155,11 @@ class MhdSolver2D {
   int low_order_ = 0;           // 1 while the positivity controller runs low order
   int last_substeps_ = 0;
   cudaGraphExec_t graph_[2] = {nullptr, nullptr};
+  // The host-driven loop's two halves, cfl_limit and step_unchecked, per
+  // parity of the live register; captured after 32 steps.
+  cudaGraphExec_t api_front_[2] = {nullptr, nullptr}, api_finish_[2] = {nullptr, nullptr};
+  int api_steps_ = 0;
+  double* dt_host_ = nullptr;  // pinned: the step's dt on its way to ctl_->dt
   void release_graphs();
   void reconstruct_stage(const StageArgs& a, int order);
   // learned mode
