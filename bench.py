@@ -348,6 +348,8 @@ def main():
                 "frac": (achieved / peak.value) if achieved else None, "traffic": traffic,
                 "peak_source": "FP64 FMA probe on this GPU (qmhd_fp64_fma_peak); "
                                "MEASURED_PEAKS.json holds no FP64 figure",
+                "note": "FLOPs of the formulas for every zone; faces in uniform gas are "
+                        "finished without them, so frac can exceed 1 on this workload",
                 "step_flop_per_zone": step_flops,
                 "step_achieved_tflops": (step_flops * value / WORLD / 1e12) if step_flops else None,
                 "phase_ms_per_step": {k: round(v, 4) for k, v in phase_ms.items()}}
