@@ -948,6 +948,7 @@ __device__ void mp_faces_warp(const Grid& g, const StateP& u, const IfaceP& out,
   }
   const unsigned vmask = __ballot_sync(0xffffffffu, valid);
   const unsigned smask = __ballot_sync(0xffffffffu, sure);
+  __syncwarp();  // the records are written (a ballot orders no memory)
   // phase 2: eight faces per round, four lanes per face
   const int gi = int(lane >> 2), rl = int(lane & 3u);
   double* grp = ws + kRec * kRecS + gi * kGrpDoubles;
