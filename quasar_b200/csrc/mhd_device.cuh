@@ -110,7 +110,8 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
   const double e = fma(-(x * y), y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
-// sqrt of x >= 0 (x below the normal range: 0)
+// sqrt of finite x >= 0 (x below the normal range: 0).  Infinity gives NaN, as
+// infinity times its inverse root: a caller whose operand can overflow tests it.
 __device__ __forceinline__ double sqrt_nr(double x) {
   const double s = x * rsqrt_nr(x);
   return x < kTiny ? 0.0 : s;
@@ -563,7 +564,9 @@ __device__ __forceinline__ Fx hlld_flux_x(const St& L, const St& R, double gamma
     return 0.5 * ((a2 + n2 + b2) + sqrt_nr(d * d + 4.0 * a2 * b2));
   };
   const double fL = fast2(pL, irl, btL2), fR = fast2(pR, irr, btR2);
-  const double cf = sqrt_nr(fL > fR ? fL : fR);
+  // an overflowing discriminant leaves NaN on its side, which a maximum would
+  // drop: infinite wave speeds, which only the HLL exit takes
+  const double cf = fL < kInf && fR < kInf ? sqrt_nr(fL > fR ? fL : fR) : kInf;
   const double sl = (vxL < vxR ? vxL : vxR) - cf, sr = (vxL > vxR ? vxL : vxR) + cf;
   if (sl >= 0.0 || sr <= 0.0) {
     const bool l = sl >= 0.0;

@@ -1541,6 +1541,8 @@ __device__ __forceinline__ Spd speed_parts(const St& s, double gamma) {
 template <int DIR, int ORDER>
 __device__ __forceinline__ double face_rate(const St& l, const St& r, double gamma, double h) {
   const Spd a = speed_parts<DIR>(l, gamma), b = speed_parts<DIR>(r, gamma);
+  // a side whose discriminant overflows has NaN here, which a maximum would drop
+  if (!(a.f2 < kInf && b.f2 < kInf)) return kInf;
   const double rate = ORDER <= 1 ? fmax(a.v + sqrt_nr(a.f2), b.v + sqrt_nr(b.f2))
                                  : fmax(a.v, b.v) + sqrt_nr(fmax(a.f2, b.f2));
   if (!(isfinite(rate) && rate >= 0.0)) return kInf;
