@@ -143,9 +143,13 @@ struct PlainDiv {
 // Processor", 1990) and four FP64 instructions a quotient: q0 = RN(a yl + RN(a
 // y)), yl the remainder of y, is within an ulp of a / b, its residual a - b q0
 // is exact, and RN(q0 + (a - b q0) y) is then the correctly rounded quotient
-// (theorem 7.1 there).  A divisor outside 2^-900 .. 2^900 sets `bad`: the
-// caller repeats the work with PlainDiv.  A numerator below 1e-291 may come
-// out an ulp off, in sums that hold a term of order one.
+// (theorem 7.1 there).  The theorem leaves out one significand, all ones,
+// whose reciprocal the corrections may leave an ulp off; from the hardware's
+// approximation they do not, and the quotients are those of division
+// (tests/test_gpu_step_math.py covers that significand).  A divisor outside
+// 2^-900 .. 2^900 sets `bad`: the caller repeats the work with PlainDiv.  A
+// numerator below 1e-291 may come out an ulp off, in sums that hold a term of
+// order one.
 struct SharedDiv {
   bool bad = false;
   struct By {
