@@ -2558,11 +2558,10 @@ __device__ __forceinline__ void b_cell_emf_s(const Grid& g, const StateP& u, dou
       for (int qy = 0; qy < Q; ++qy) row[qy] = gauss_avg<ORDER>(pt[qy]);
       e = gauss_avg<ORDER>(row);
     } else if (uniform) {
-      // what its points give, bit for bit; the staged state, not the register's
+      // what its points give, bit for bit: the same correctly rounded 1 / rho,
+      // whether they are admissible or not; the staged state, not the register's
       auto at = [&](int c) { return S[c * SY * RS + XO]; };
-      const St c{at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7)};
-      const double ir = rcp_nr(c.rho);
-      e = point_admissible_ir(c, gamma, ir) ? physical_ez_ir(c, ir) : physical_ez(c);
+      e = physical_ez(St{at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7)});
     } else {
       e = physical_ez(load_cell(u, k));
     }
