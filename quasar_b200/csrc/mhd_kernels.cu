@@ -2608,21 +2608,34 @@ __global__ void __launch_bounds__(256, 3) k_cell_emf_tma(Grid g, StateP u,
 // reference's constant shortcut); *cst, where asked for, is whether they are.
 template <int NT>
 __device__ __forceinline__ double edge_interp(const double* e, bool* cst = nullptr) {
+  if (NT == 2) {
+    if (cst) *cst = e[0] == e[1];
+    return __dmul_rn(__dadd_rn(e[0], e[1]), 0.5);  // = / 2 exactly
+  }
   double d[NT];
   unsigned bits = 0u;
 #pragma unroll
   for (int q = 1; q < NT; ++q) {
     d[q] = __dsub_rn(e[q], e[0]);
-    // +0 only where the samples are equal (NaN and infinities differ)
-    bits |= unsigned(__double2hiint(d[q])) | unsigned(__double2loint(d[q]));
+    // a zero of either sign only where finite samples are equal
+    bits |= (unsigned(__double2hiint(d[q])) & 0x7fffffffu) | unsigned(__double2loint(d[q]));
   }
-  if (cst) *cst = bits == 0u;
-  if (NT == 2) return fma(0.5, d[1], e[0]);
+  double r;
   if (NT == 6)
-    return fma(1.0 / 60.0, fma(37.0, d[2] + d[3], fma(-8.0, d[1] + d[4], d[5])), e[0]);
-  return fma(1.0 / 840.0,
-             fma(533.0, d[3] + d[4], -139.0 * (d[2] + d[5])) + fma(29.0, d[1] + d[6], -3.0 * d[7]),
-             e[0]);
+    r = fma(1.0 / 60.0, fma(37.0, d[2] + d[3], fma(-8.0, d[1] + d[4], d[5])), e[0]);
+  else
+    r = fma(1.0 / 840.0,
+            fma(533.0, d[3] + d[4], -139.0 * (d[2] + d[5])) + fma(29.0, d[1] + d[6], -3.0 * d[7]),
+            e[0]);
+  bool same = bits == 0u;
+  if (r != r) {  // equal infinities differ by NaN and return their value
+    same = true;
+#pragma unroll
+    for (int q = 1; q < NT; ++q) same = same && e[q] == e[0];
+    if (same) r = e[0];
+  }
+  if (cst) *cst = same;
+  return r;
 }
 
 // Upwind CT corner E_z = ex + ey - centred, with the exact one-dimensional
