@@ -422,8 +422,11 @@ __device__ __forceinline__ double mp_curvature(double p, double q) {
 // only its round-off form is tested, |cc| |cm| <= 1e-10 var^2.  Of var's
 // four terms the two differences suffice: |cc| or |cm| is the largest only
 // where cc or cm is within 1e-10 of zero relative to a difference, and there
-// the limited and the unlimited value agree to that.  Returns the limited
-// offset.  NaN offsets compare false and are returned.
+// the limited and the unlimited value agree to that.  An offset whose square
+// would leave the binary64 range (below 2^-480, from 2^490) is first scaled, with
+// the differences, by a power of two, so that the test is the same at every
+// magnitude.  Returns the limited offset.  NaN offsets compare false and are
+// returned.
 __device__ __forceinline__ double mp_side(double cc, double dpl, double dmn, double md,
                                           double lc) {
   const int s = __double2hiint(cc) & 0x80000000;
@@ -435,9 +438,18 @@ __device__ __forceinline__ double mp_side(double cc, double dpl, double dmn, dou
   bound = __double2hiint(bound) < 0 ? 0.0 : bound;
   double mm = fabs(d) < fabs(ul) ? d : ul;
   mm = (__double2hiint(d) ^ __double2hiint(ul)) < 0 ? 0.0 : mm;
-  const double P = ac * (ac - mm) * 1e10;
-  const int above = __double2hiint(fma(dmn, dmn, -P)) & __double2hiint(fma(dpl, dpl, -P));
-  return ac > bound && above < 0 ? flip_sign(bound, s) : cc;
+  if (!(ac > bound)) return cc;
+  double x = ac, y = ac - mm, p = dpl, q = dmn;
+  if (unsigned(__double2hiint(ac)) - (543u << 20) >= 970u << 20) {
+    const double z = __hiloint2double(__double2hiint(ac) < (543 << 20) ? 1623 << 20 : 423 << 20, 0);
+    x *= z;
+    y *= z;
+    p *= z;
+    q *= z;
+  }
+  const double P = x * y * 1e10;
+  const int above = __double2hiint(fma(q, q, -P)) & __double2hiint(fma(p, p, -P));
+  return above < 0 ? flip_sign(bound, s) : cc;
 }
 // The MP5 / MP7 face values on both sides of the face between samples H and
 // H + 1 of c[0 .. 2H + 1] (mp_limiter.hpp:71-224 for the window and its
