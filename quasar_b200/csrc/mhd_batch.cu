@@ -1,5 +1,6 @@
 // Batched MHD step (see mhd_batch.cuh).
 #include "mhd_batch.cuh"
+#include "graph_capture.cuh"
 #include "indicator.cuh"
 
 #include <algorithm>
@@ -243,19 +244,8 @@ void MhdBatch2D::enqueue_step(int par, std::vector<cudaEvent_t>* marks,
 
 void MhdBatch2D::ensure_graphs() {
   if (graph_[0]) return;
-  for (int par = 0; par < 2; ++par) {
-    cudaGraph_t g;
-    ck(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture");
-    try {
-      enqueue_step(par, nullptr, nullptr);
-    } catch (...) {
-      cudaStreamEndCapture(stream_, &g);
-      throw;
-    }
-    ck(cudaStreamEndCapture(stream_, &g), "capture end");
-    ck(cudaGraphInstantiate(&graph_[par], g, 0), "graph instantiate");
-    cudaGraphDestroy(g);
-  }
+  ck(capture_graphs(stream_, 2, [&](int par) { enqueue_step(par, nullptr, nullptr); }, graph_),
+     "step graphs");
 }
 
 void MhdBatch2D::release_graphs() {

@@ -3,6 +3,7 @@
 // MhdSolver2D (src/physics/mhd/mhd_solver.cpp) call for call where the
 // semantics are observable: preflights, CFL cap, retry policy, errors.
 #include "mhd_solver.cuh"
+#include "graph_capture.cuh"
 #include "indicator.cuh"
 
 #include <cuda.h>
@@ -378,11 +379,12 @@ StageArgs MhdSolver2D::live_args() {
 }
 
 void MhdSolver2D::release_graphs() {
-  for (cudaGraphExec_t* set : {graph_, api_front_, api_finish_})
-    for (int k = 0; k < 2; ++k) {
-      if (set[k]) cudaGraphExecDestroy(set[k]);
-      set[k] = nullptr;
-    }
+  auto release = [](cudaGraphExec_t& e) {
+    if (e) cudaGraphExecDestroy(e);
+    e = nullptr;
+  };
+  for (auto& e : graph_) release(e);
+  for (auto& e : api_graph_) release(e);
   api_steps_ = 0;
 }
 
@@ -504,7 +506,7 @@ double MhdSolver2D::cfl_limit_for(int coll) {
   const int order = coll > 0 ? 1 : cfg_.order;
   if (front_order_ != order || front_dt_mode_ == 0) {
     if (coll == 0 && anchor_mode_ == -1 && api_graphs())
-      ck(cudaGraphLaunch(api_front_[live_ == 0 ? 0 : 1], stream_), "graph launch");
+      ck(cudaGraphLaunch(api_graph_[live_ == 0 ? 0 : 2], stream_), "graph launch");
     else
       front_impl(order, 1, anchor_mode_);
     front_order_ = order;
@@ -572,7 +574,7 @@ void MhdSolver2D::advance_positive(double dt) {
   if (api_graphs()) {
     *dt_host_ = dt;  // the last step's copy has completed: every step ends with read_ctl
     ck(cudaMemcpyAsync(&ctl_->dt, dt_host_, sizeof(double), cudaMemcpyHostToDevice, stream_), "dt");
-    ck(cudaGraphLaunch(api_finish_[live_ == 0 ? 0 : 1], stream_), "graph launch");
+    ck(cudaGraphLaunch(api_graph_[live_ == 0 ? 1 : 3], stream_), "graph launch");
   } else {
     finish_impl(cfg_.order, nullptr, dt, false);
   }
@@ -711,24 +713,31 @@ void MhdSolver2D::conserved_cell_totals(double* mass, double* energy) {
   *energy = double(e);
 }
 
+// The registers' roles, given back also when a capture fails.
+struct MhdSolver2D::KeepRoles {
+  MhdSolver2D& s;
+  int live = s.live_, next = s.next_;
+  ~KeepRoles() {
+    s.live_ = live;
+    s.next_ = next;
+  }
+  void parity(int k) {
+    s.live_ = k == 0 ? 0 : 3;
+    s.next_ = k == 0 ? 3 : 0;
+  }
+};
+
 // One graph per register assignment: a complete auto-dt step from the live
 // register into the next one (the roles swap each accepted step).
 void MhdSolver2D::build_graphs() {
   if (graph_[0]) return;
-  const int keep_live = live_, keep_next = next_;
-  for (int k = 0; k < 2; ++k) {
-    live_ = k == 0 ? 0 : 3;
-    next_ = k == 0 ? 3 : 0;
-    cudaGraph_t graph;
-    ck(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture");
-    front_impl(cfg_.order, 2, -1);
-    finish_impl(cfg_.order, &ctl_->dt, 0.0, true);
-    ck(cudaStreamEndCapture(stream_, &graph), "capture end");
-    ck(cudaGraphInstantiate(&graph_[k], graph, 0), "graph instantiate");
-    cudaGraphDestroy(graph);
-  }
-  live_ = keep_live;
-  next_ = keep_next;
+  KeepRoles roles{*this};
+  ck(capture_graphs(stream_, 2, [&](int k) {
+       roles.parity(k);
+       front_impl(cfg_.order, 2, -1);
+       finish_impl(cfg_.order, &ctl_->dt, 0.0, true);
+     }, graph_),
+     "step graphs");
 }
 
 // The host-driven loop (cfl_limit, step_unchecked) as graph replays: its 24
@@ -736,34 +745,27 @@ void MhdSolver2D::build_graphs() {
 // MP5: 0.31 -> 0.26 ms per step).  The capture costs what eight steps save; it
 // is made after 32 steps, so that a loop that ends just there loses 4%.
 // False until then (counted from construction or a change of the window), and
-// with an indicator, whose network may be trained on between two steps.
+// with an indicator, whose network may be trained on between two steps.  The
+// loop needs no graph: one that cannot be made (no memory left) leaves it at
+// its launches, and is tried again 32 steps later.
 bool MhdSolver2D::api_graphs() {
   if (ind_ || marks_) return false;
-  if (api_finish_[1]) return true;
+  if (api_graph_[0]) return true;
   if (api_steps_ <= 32) return false;
-  struct Keep {  // the registers' roles, also when a capture fails
-    MhdSolver2D& s;
-    int live, next;
-    ~Keep() {
-      s.live_ = live;
-      s.next_ = next;
-    }
-  } keep{*this, live_, next_};
-  for (int k = 0; k < 2; ++k) {
-    live_ = k == 0 ? 0 : 3;
-    next_ = k == 0 ? 3 : 0;
-    for (int half = 0; half < 2; ++half) {
-      cudaGraph_t graph;
-      ck(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture");
-      if (half == 0) front_impl(cfg_.order, 1, -1);
+  KeepRoles roles{*this};
+  try {
+    const cudaError_t e = capture_graphs(stream_, 4, [&](int k) {
+      roles.parity(k / 2);
+      if (k % 2 == 0) front_impl(cfg_.order, 1, -1);
       else finish_impl(cfg_.order, &ctl_->dt, 0.0, false);
-      ck(cudaStreamEndCapture(stream_, &graph), "capture end");
-      ck(cudaGraphInstantiate(half == 0 ? &api_front_[k] : &api_finish_[k], graph, 0),
-         "graph instantiate");
-      cudaGraphDestroy(graph);
-    }
+    }, api_graph_);
+    if (e == cudaSuccess) return true;
+  } catch (const CudaError&) {
+    // a lasting error meets the launches that follow
   }
-  return true;
+  cudaGetLastError();
+  api_steps_ = 0;
+  return false;
 }
 
 int MhdSolver2D::advance_auto(double* t_io, double t_end, int max_steps) {

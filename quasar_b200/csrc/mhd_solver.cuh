@@ -157,7 +157,8 @@ class MhdSolver2D {
   cudaGraphExec_t graph_[2] = {nullptr, nullptr};
   // The host-driven loop's two halves, cfl_limit and step_unchecked, per
   // parity of the live register; captured after 32 steps.
-  cudaGraphExec_t api_front_[2] = {nullptr, nullptr}, api_finish_[2] = {nullptr, nullptr};
+  cudaGraphExec_t api_graph_[4] = {nullptr, nullptr, nullptr, nullptr};
+  struct KeepRoles;
   int api_steps_ = 0;
   double* dt_host_ = nullptr;  // pinned: the step's dt on its way to ctl_->dt
   void release_graphs();
