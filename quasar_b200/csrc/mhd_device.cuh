@@ -97,12 +97,24 @@ __device__ __forceinline__ double div_by(double x, double h, double rh) {
 // instructions and no branch, where the correctly rounded forms take twice
 // as many and a test for the exceptional operands.  For results that depend
 // continuously on rounding, x normal and positive or negative (square root:
-// positive); subnormal, infinite and NaN operands give a non-finite value.
+// positive); subnormal, infinite and NaN operands give a non-finite value, and
+// the reciprocal is zero from 2^1022 on.
 __device__ __forceinline__ double rcp_nr(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-x, y, 1.0);
   return fma(y, fma(e, e, e), y);
+}
+// Densities below the normal range are admissible too, but rcp_nr has NaN for
+// them, which every admissibility test refuses; the last resort of each kernel
+// (first-order face states, the face-average Riemann problem and its speeds)
+// scales them by a power of two.
+__device__ __forceinline__ bool subnormal(double x) {
+  return unsigned(__double2hiint(x)) < 0x00100000u;
+}
+__device__ __forceinline__ double rcp_rho(double x) {
+  const double z = subnormal(x) ? 0x1p64 : 1.0;
+  return rcp_nr(x * z) * z;
 }
 __device__ __forceinline__ double rsqrt_nr(double x) {
   double y;
@@ -310,6 +322,15 @@ __device__ __forceinline__ bool point_admissible_ir(const St& s, double gamma, d
 }
 __device__ __forceinline__ bool point_admissible(const St& s, double gamma) {
   return point_admissible_ir(s, gamma, rcp_nr(s.rho));
+}
+
+// The same for a density below the normal range: 2 rho (E - B^2 / 2) > m^2 with
+// density, energy and momentum scaled by 2^1000.
+__device__ __forceinline__ bool subnormal_admissible(const St& s) {
+  constexpr double z = 0x1p1000;
+  const double q = 2.0 * (s.E - 0.5 * (s.bx * s.bx + s.by * s.by + s.bz * s.bz));
+  const double mx = s.mx * z, my = s.my * z, mz = s.mz * z;
+  return subnormal(s.rho) && q < kInf && (s.rho * z) * (q * z) > mx * mx + my * my + mz * mz;
 }
 
 __device__ __forceinline__ bool recon_admissible(const St& s, double gamma) {

@@ -1297,7 +1297,8 @@ __device__ __forceinline__ void finish_face(const Grid& g, const StateP& u, cons
     set_normal_b<DIR>(ul, bn);
     set_normal_b<DIR>(ur, bn);
   }
-  if (!recon_admissible(ul, gamma) || !recon_admissible(ur, gamma)) {
+  if (!(recon_admissible(ul, gamma) || subnormal_admissible(ul)) ||
+      !(recon_admissible(ur, gamma) || subnormal_admissible(ur))) {
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
     ul = St{nan, nan, nan, nan, nan, nan, nan, nan};
     ur = ul;
@@ -1516,7 +1517,7 @@ struct Spd {
   double v, f2;
 };
 
-// One side's |v_n| and squared fast speed (mhd_reduce.hip:254-325), with one
+// One side's |v_n| and squared fast speed (mhd_reduce.hip:254-325), with the
 // reciprocal of rho.  The discriminant is formed as (a^2 - b^2)^2 + 4 a^2 b_t^2,
 // which equals the reference's (a^2 + b^2)^2 - 4 a^2 b_n^2 but has no
 // cancellation: where the reference's rounding is amplified to sqrt(eps) (a
@@ -1524,8 +1525,7 @@ struct Spd {
 // ulps, and elsewhere both agree to rounding.  A non-finite component makes
 // the pressure fail its test (point_admissible_p).
 template <int DIR>
-__device__ __forceinline__ Spd speed_parts(const St& s, double gamma) {
-  const double ir = rcp_nr(s.rho);
+__device__ __forceinline__ Spd speed_parts(const St& s, double gamma, double ir) {
   const double p = pressure_f(s, gamma, ir);
   if (!point_admissible_p(s, p)) return Spd{kInf, kInf};
   const double bn = DIR == 0 ? s.bx : s.by, b1 = DIR == 0 ? s.by : s.bx;
@@ -1539,8 +1539,9 @@ __device__ __forceinline__ Spd speed_parts(const St& s, double gamma) {
 
 // Weighted face rate 0.5*alpha/h of one Riemann problem (mhd_reduce.hip:331-383).
 template <int DIR, int ORDER>
-__device__ __forceinline__ double face_rate(const St& l, const St& r, double gamma, double h) {
-  const Spd a = speed_parts<DIR>(l, gamma), b = speed_parts<DIR>(r, gamma);
+__device__ __forceinline__ double face_rate(const St& l, const St& r, double gamma, double h,
+                                            double irl, double irr) {
+  const Spd a = speed_parts<DIR>(l, gamma, irl), b = speed_parts<DIR>(r, gamma, irr);
   // a side whose discriminant overflows has NaN here, which a maximum would drop
   if (!(a.f2 < kInf && b.f2 < kInf)) return kInf;
   const double rate = ORDER <= 1 ? fmax(a.v + sqrt_nr(a.f2), b.v + sqrt_nr(b.f2))
@@ -1577,7 +1578,7 @@ __global__ void __launch_bounds__(128) k_face_flux(Grid g, IfaceP in, FluxP out,
   constexpr bool kLF = ORDER <= 1;
   if (ORDER != 5 && ORDER != 7) {
     f = riemann<DIR>(bl, br, kLF, gamma);
-    if (spd) rate = face_rate<DIR, ORDER>(bl, br, gamma, h);
+    if (spd) rate = face_rate<DIR, ORDER>(bl, br, gamma, h, rcp_rho(bl.rho), rcp_rho(br.rho));
   } else {
     constexpr int H = ORDER == 5 ? 2 : 3, N = 2 * H + 1, Q = ORDER == 5 ? 3 : 4;
     const long long ts = DIR == 0 ? g.pitch : 1;
@@ -1610,11 +1611,11 @@ __global__ void __launch_bounds__(128) k_face_flux(Grid g, IfaceP in, FluxP out,
       }
     }
     if (spd) {
-      rate = face_rate<DIR, ORDER>(bl, br, gamma, h);
+      rate = face_rate<DIR, ORDER>(bl, br, gamma, h, rcp_rho(bl.rho), rcp_rho(br.rho));
       for (int q = 0; q < first_bad; ++q) {
         const St l{pl[q][0], pl[q][1], pl[q][2], pl[q][3], pl[q][4], pl[q][5], pl[q][6], pl[q][7]};
         const St r{pr[q][0], pr[q][1], pr[q][2], pr[q][3], pr[q][4], pr[q][5], pr[q][6], pr[q][7]};
-        rate = fmax(rate, face_rate<DIR, ORDER>(l, r, gamma, h));
+        rate = fmax(rate, face_rate<DIR, ORDER>(l, r, gamma, h, rcp_rho(l.rho), rcp_rho(r.rho)));
       }
     }
     if (!ok) {
@@ -1775,7 +1776,7 @@ __device__ __forceinline__ void constant_tile_flux(const Grid& g, const FluxP& o
   if (f >= TX * TY || i > g.nx || j > g.ny) return;
   const long long k = g.idx(i, j);
   const St u{at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7)};
-  const double ir = rcp_nr(u.rho);
+  const double ir = rcp_rho(u.rho);
   const Fx v = flat_flux<DIR>(u, pressure_f(u, gamma, ir), ir);
   if (out.f[0]) {
     out.f[0][k] = v.rho;
@@ -1788,7 +1789,7 @@ __device__ __forceinline__ void constant_tile_flux(const Grid& g, const FluxP& o
     out.f[7][k] = v.bz;
   }
   if (emf) emf[k] = DIR == 0 ? -v.by : v.bx;
-  if (spd) spd[k] = face_rate<DIR, ORDER>(u, u, gamma, DIR == 0 ? g.dx : g.dy);
+  if (spd) spd[k] = face_rate<DIR, ORDER>(u, u, gamma, DIR == 0 ? g.dx : g.dy, ir, ir);
   if (nj) nj[k] = 1;
 }
 
@@ -1900,15 +1901,18 @@ __device__ __forceinline__ void b_face_flux_pt(const Grid& g, const IfaceP& in, 
   const int first_bad = bad ? __ffs(bad) - 1 : Q;
   double rate = 0.0;
   if (spd) {
-    if (lane == 0) rate = face_rate<DIR, ORDER>(centre(true), centre(false), gamma, h);
-    if (lane < first_bad) rate = fmax(rate, face_rate<DIR, ORDER>(l, r, gamma, h));
+    if (lane == 0) {
+      const St a = centre(true), b = centre(false);
+      rate = face_rate<DIR, ORDER>(a, b, gamma, h, rcp_rho(a.rho), rcp_rho(b.rho));
+    }
+    if (lane < first_bad) rate = fmax(rate, face_rate<DIR, ORDER>(l, r, gamma, h, irl, irr));
   }
   const bool solve = group_ok || lane == 0;
   if (!group_ok) {
     l = centre(true);
     r = centre(false);
-    irl = rcp_nr(l.rho);
-    irr = rcp_nr(r.rho);
+    irl = rcp_rho(l.rho);
+    irr = rcp_rho(r.rho);
     prl = pressure_f(l, gamma, irl);
     prr = pressure_f(r, gamma, irr);
   }
@@ -2107,15 +2111,18 @@ __device__ __forceinline__ void b_face_flux_cs(const Grid& g, const IfaceP& in, 
   const int first_bad = bad ? __ffs(bad) - 1 : Q;
   double rate = 0.0;
   if (spd) {
-    if (lane == 0) rate = face_rate<DIR, ORDER>(centre(true), centre(false), gamma, h);
-    if (lane < first_bad) rate = fmax(rate, face_rate<DIR, ORDER>(l, r, gamma, h));
+    if (lane == 0) {
+      const St a = centre(true), b = centre(false);
+      rate = face_rate<DIR, ORDER>(a, b, gamma, h, rcp_rho(a.rho), rcp_rho(b.rho));
+    }
+    if (lane < first_bad) rate = fmax(rate, face_rate<DIR, ORDER>(l, r, gamma, h, irl, irr));
   }
   const bool solve = group_ok || lane == 0;
   if (!group_ok) {
     l = centre(true);
     r = centre(false);
-    irl = rcp_nr(l.rho);
-    irr = rcp_nr(r.rho);
+    irl = rcp_rho(l.rho);
+    irr = rcp_rho(r.rho);
     prl = pressure_f(l, gamma, irl);
     prr = pressure_f(r, gamma, irr);
   }
@@ -4205,7 +4212,8 @@ __device__ double abi_face_rate(const Grid& g, const IfaceP& in, int i, int j, d
   if (DIR == 1 && j == g.ny && g.bc[2] == 0 && g.bc[3] == 0) sj = 0;
   const long long ks = g.idx(si, sj);
   const double h = DIR == 0 ? g.dx : g.dy;
-  double rate = face_rate<DIR, ORDER>(iface(in, ks, true), iface(in, ks, false), gamma, h);
+  const St bl = iface(in, ks, true), br = iface(in, ks, false);
+  double rate = face_rate<DIR, ORDER>(bl, br, gamma, h, rcp_rho(bl.rho), rcp_rho(br.rho));
   if (ORDER != 5 && ORDER != 7) return rate;
   constexpr int H = ORDER == 5 ? 2 : 3, N = 2 * H + 1, Q = ORDER == 5 ? 3 : 4;
   const long long ts = DIR == 0 ? g.pitch : 1;
@@ -4234,7 +4242,7 @@ __device__ double abi_face_rate(const Grid& g, const IfaceP& in, int i, int j, d
     const St l{pl[0], pl[1], pl[2], pl[3], pl[4], pl[5], pl[6], pl[7]};
     const St r{pr[0], pr[1], pr[2], pr[3], pr[4], pr[5], pr[6], pr[7]};
     if (!point_admissible(l, gamma) || !point_admissible(r, gamma)) break;
-    rate = fmax(rate, face_rate<DIR, ORDER>(l, r, gamma, h));
+    rate = fmax(rate, face_rate<DIR, ORDER>(l, r, gamma, h, rcp_nr(l.rho), rcp_nr(r.rho)));
   }
   return rate;
 }
