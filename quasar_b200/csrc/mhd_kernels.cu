@@ -1558,6 +1558,8 @@ __device__ __forceinline__ St iface(const IfaceP& v, long long k, bool left) {
             __ldg(v.R[4] + k), __ldg(v.R[5] + k), __ldg(v.R[6] + k), __ldg(v.R[7] + k)};
 }
 
+// Orders 1 and 2, whose face states need no transverse quadrature: one thread
+// per face.
 template <int DIR, int ORDER>
 __global__ void __launch_bounds__(128) k_face_flux(Grid g, IfaceP in, FluxP out, double* emf,
                                                    int* nj, double* spd, double gamma,
@@ -1571,77 +1573,8 @@ __global__ void __launch_bounds__(128) k_face_flux(Grid g, IfaceP in, FluxP out,
   if (DIR == 0 && i == g.nx && g.bc[0] == 0 && g.bc[1] == 0) si = 0;
   if (DIR == 1 && j == g.ny && g.bc[2] == 0 && g.bc[3] == 0) sj = 0;
   const long long k = g.idx(i, j), ks = g.idx(si, sj);
-  const double h = DIR == 0 ? g.dx : g.dy;
   const St bl = iface(in, ks, true), br = iface(in, ks, false);
-  Fx f;
-  double rate = 0.0;
-  constexpr bool kLF = ORDER <= 1;
-  if (ORDER != 5 && ORDER != 7) {
-    f = riemann<DIR>(bl, br, kLF, gamma);
-    if (spd) rate = face_rate<DIR, ORDER>(bl, br, gamma, h, rcp_rho(bl.rho), rcp_rho(br.rho));
-  } else {
-    constexpr int H = ORDER == 5 ? 2 : 3, N = 2 * H + 1, Q = ORDER == 5 ? 3 : 4;
-    const long long ts = DIR == 0 ? g.pitch : 1;
-    // Recover the Q Gauss-point states of both sides from N transverse face
-    // averages (mhd_face_quadrature.hpp:114-142).
-    double pl[Q][8], pr[Q][8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      double sa[N], sb[N];
-#pragma unroll
-      for (int t = 0; t < N; ++t) {
-        sa[t] = __ldg(in.L[c] + ks + (t - H) * ts);
-        sb[t] = __ldg(in.R[c] + ks + (t - H) * ts);
-      }
-#pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        pl[q][c] = point_value<ORDER>(q, sa);
-        pr[q][c] = point_value<ORDER>(q, sb);
-      }
-    }
-    bool ok = true;
-    int first_bad = Q;
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const St l{pl[q][0], pl[q][1], pl[q][2], pl[q][3], pl[q][4], pl[q][5], pl[q][6], pl[q][7]};
-      const St r{pr[q][0], pr[q][1], pr[q][2], pr[q][3], pr[q][4], pr[q][5], pr[q][6], pr[q][7]};
-      if (!point_admissible(l, gamma) || !point_admissible(r, gamma)) {
-        ok = false;
-        if (first_bad == Q) first_bad = q;
-      }
-    }
-    if (spd) {
-      rate = face_rate<DIR, ORDER>(bl, br, gamma, h, rcp_rho(bl.rho), rcp_rho(br.rho));
-      for (int q = 0; q < first_bad; ++q) {
-        const St l{pl[q][0], pl[q][1], pl[q][2], pl[q][3], pl[q][4], pl[q][5], pl[q][6], pl[q][7]};
-        const St r{pr[q][0], pr[q][1], pr[q][2], pr[q][3], pr[q][4], pr[q][5], pr[q][6], pr[q][7]};
-        rate = fmax(rate, face_rate<DIR, ORDER>(l, r, gamma, h, rcp_rho(l.rho), rcp_rho(r.rho)));
-      }
-    }
-    if (!ok) {
-      // A transverse polynomial may leave the admissible set: fall back to the
-      // face-average problem (mhd_face_quadrature.hpp:234-239).
-      f = riemann<DIR>(bl, br, kLF, gamma);
-    } else {
-      double fq[8][Q];
-#pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        const St l{pl[q][0], pl[q][1], pl[q][2], pl[q][3], pl[q][4], pl[q][5], pl[q][6], pl[q][7]};
-        const St r{pr[q][0], pr[q][1], pr[q][2], pr[q][3], pr[q][4], pr[q][5], pr[q][6], pr[q][7]};
-        const Fx fl = riemann<DIR>(l, r, kLF, gamma);
-        fq[0][q] = fl.rho; fq[1][q] = fl.mx; fq[2][q] = fl.my; fq[3][q] = fl.mz;
-        fq[4][q] = fl.E;   fq[5][q] = fl.bx; fq[6][q] = fl.by; fq[7][q] = fl.bz;
-      }
-      f.rho = gauss_avg<ORDER>(fq[0]);
-      f.mx = gauss_avg<ORDER>(fq[1]);
-      f.my = gauss_avg<ORDER>(fq[2]);
-      f.mz = gauss_avg<ORDER>(fq[3]);
-      f.E = gauss_avg<ORDER>(fq[4]);
-      f.bx = gauss_avg<ORDER>(fq[5]);
-      f.by = gauss_avg<ORDER>(fq[6]);
-      f.bz = gauss_avg<ORDER>(fq[7]);
-    }
-  }
+  const Fx f = riemann<DIR>(bl, br, ORDER <= 1, gamma);
   // out, emf and nj may each be absent (the per-kernel launch interface
   // asks for fluxes or for the CT face tables alone)
   if (out.f[0]) {
@@ -1656,24 +1589,18 @@ __global__ void __launch_bounds__(128) k_face_flux(Grid g, IfaceP in, FluxP out,
   }
   // Directional Godunov E_z: F_x(By) = -Ez, F_y(Bx) = +Ez (mhd_ct.hip:126-133).
   if (emf) emf[k] = DIR == 0 ? -f.by : f.bx;
-  if (spd) spd[k] = rate;
+  if (spd)
+    spd[k] = face_rate<DIR, ORDER>(bl, br, gamma, DIR == 0 ? g.dx : g.dy, rcp_rho(bl.rho),
+                                   rcp_rho(br.rho));
   if (!nj) return;
-  // "No jump" proof of the complete point-recovered problem
-  // (mhd_ct.hip:150-174); taps are mapped like every CT table read.
-  constexpr int RH = ORDER >= 7 ? 3 : ORDER >= 5 ? 2 : 0;
+  // "No jump" proof of the face's problem (mhd_ct.hip:150-174), mapped like
+  // every CT table read.
+  const long long km = g.idx(face_index(i, g.nx, g.bc[0], g.bc[1]),
+                             face_index(j, g.ny, g.bc[2], g.bc[3]));
   int proof = 1;
-  for (int off = -RH; off <= RH && proof; ++off) {
-    const int mi = face_index(DIR == 0 ? i : i + off, g.nx, g.bc[0], g.bc[1]);
-    const int mj = face_index(DIR == 0 ? j + off : j, g.ny, g.bc[2], g.bc[3]);
-    if (!in_pad(g, mi, mj)) {
-      proof = 0;
-      break;
-    }
-    const long long km = g.idx(mi, mj);
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
-      if (!(in.L[c][km] == in.R[c][km])) proof = 0;
-  }
+  for (int c = 0; c < 8; ++c)
+    if (!(in.L[c][km] == in.R[c][km])) proof = 0;
   nj[k] = proof;
 }
 
@@ -1687,16 +1614,13 @@ __global__ void __launch_bounds__(128) k_face_flux(Grid g, IfaceP in, FluxP out,
 // row (2.8x fewer for x faces, 4x for y faces at MP7).  At MP7 the
 // transverse recovery is split by component: lane q forms components q,
 // q + 4, ... at every Gauss point of its face (each stencil column read
-// once, and the constant-stencil shortcut, which decides the same for every
-// point, tested once per component) into the face's point rows in shared
-// memory, from which each lane takes its own point's 16 components as
-// 16-byte pairs.  Each lane solves its point's Riemann problem, the group
+// once) into the face's point rows in shared memory, from which each lane
+// takes its own point's 16 components as 16-byte pairs.  Each lane solves its point's Riemann problem, the group
 // votes on admissibility, and the point fluxes go back through the same
 // rows, where lane q forms and stores the Gauss sums of components q, q + 4
 // (rotor 4096^2 MP7: face flux 27.6 -> 23.3 ms per step; Orszag-Tang 2048^2
 // MP7: 10.8 -> 10.4).  At MP5 each lane recovers its own point (below).
-// Same sums in the same node order as k_face_flux; the compiler's fused
-// multiply-adds may pair differently, a rounding-level difference.  128 threads
+// 128 threads
 // (smaller blocks than 16 x 4 measured 3-5% faster at MP7: a block waiting
 // at the staging barrier holds fewer warps).
 // ---------------------------------------------------------------------------
@@ -2292,13 +2216,13 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-// Cell-average E_z by tensor Gauss quadrature of recovered point states
-// (mhd_ct.hip:457-629); on stage 0 also the CFL max-reduction over cells
-// (mhd_reduce.hip:418-501): warp shuffles, one atomic per block.
+// Orders 1 and 2: E_z of the cell states (mhd_ct.hip:457-629); on stage 0 also
+// the CFL max-reduction over cells (mhd_reduce.hip:418-501): warp shuffles, one
+// atomic per block.
 template <int ORDER>
 __global__ void __launch_bounds__(128) k_cell_emf(Grid g, StateP u, double* cell_ez,
                                                   const double* xs, const double* ys,
-                                                  int cfl_reduce, double gamma, Ctl* ctl) {
+                                                  int cfl_reduce, Ctl* ctl) {
   __shared__ int s_stop;
   __shared__ double s_max[4];
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
@@ -2311,44 +2235,7 @@ __global__ void __launch_bounds__(128) k_cell_emf(Grid g, StateP u, double* cell
   if (i <= g.nx && j <= g.ny && !((i == g.nx && !phx) || (j == g.ny && !phy))) {
     const long long k = g.idx(i, j);
     const St c0 = ORDER <= 1 ? load_cell1(u, g, i, j) : load_cell(u, k);
-    double e = physical_ez(c0);
-    constexpr int H = ORDER >= 7 ? 3 : 2, N = 2 * H + 1, Q = ORDER >= 7 ? 4 : 3;
-    if ((ORDER == 5 || ORDER == 7) && i - H >= -g.ng && i + H <= g.nx + g.ng - 1 &&
-        j - H >= -g.ng && j + H <= g.ny + g.ng - 1) {
-      double pt[Q][Q];
-      bool ok = true;
-      const double* src[8] = {u.c[0], u.c[1], u.c[2], u.c[3], u.c[4], u.bxc, u.byc, u.c[7]};
-      for (int qx = 0; qx < Q && ok; ++qx) {
-        double rows[8][N];
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-#pragma unroll
-          for (int r = 0; r < N; ++r) {
-            double s[N];
-            const long long kr = k + (long long)(r - H) * g.pitch;
-#pragma unroll
-            for (int t = 0; t < N; ++t) s[t] = __ldg(src[c] + kr + (t - H));
-            rows[c][r] = point_value<ORDER>(qx, s);
-          }
-#pragma unroll
-        for (int qy = 0; qy < Q; ++qy) {
-          const St p{point_value<ORDER>(qy, rows[0]), point_value<ORDER>(qy, rows[1]),
-                     point_value<ORDER>(qy, rows[2]), point_value<ORDER>(qy, rows[3]),
-                     point_value<ORDER>(qy, rows[4]), point_value<ORDER>(qy, rows[5]),
-                     point_value<ORDER>(qy, rows[6]), point_value<ORDER>(qy, rows[7])};
-          const double ir = 1.0 / p.rho;
-          if (!point_admissible_ir(p, gamma, ir)) ok = false;
-          pt[qy][qx] = physical_ez_ir(p, ir);
-        }
-      }
-      if (ok) {
-        double row[Q];
-#pragma unroll
-        for (int qy = 0; qy < Q; ++qy) row[qy] = gauss_avg<ORDER>(pt[qy]);
-        e = gauss_avg<ORDER>(row);
-      }
-    }
-    cell_ez[k] = e;
+    cell_ez[k] = physical_ez(c0);
   }
   if (!cfl_reduce) return;
   double local = 0.0;
@@ -2890,7 +2777,8 @@ __device__ __forceinline__ void b_update(const Grid& g, const StateP& un, const 
 // 16-byte double2 access (the pair's first padded column is even and the
 // pitch is even, so each pair is aligned); the per-cell arithmetic and the
 // cells written are b_update's.  Reads of the pair's partner beyond the
-// updated range stay inside the padded arrays (ng >= 3).
+// updated range stay inside their padded rows from two ghost layers on: the
+// pitch, and with it nx, is even, so they end at column nx + 1, and at row ny.
 __device__ __forceinline__ double2 ld2(const double* p) {
   return __ldg(reinterpret_cast<const double2*>(p));
 }
@@ -3442,10 +3330,8 @@ void launch_cell_emf(const StageArgs& a, bool cfl_reduce, cudaStream_t s) {
   const dim3 grid(cdiv(g.nx + 1, kBX), cdiv(g.ny + 1, 4));
   const int r = cfl_reduce ? 1 : 0;
   switch (a.order) {
-    case 1: k_cell_emf<1><<<grid, block, 0, s>>>(g, a.u, a.cell_ez, a.xspd, a.yspd, r, a.gamma, a.ctl); break;
-    case 2: k_cell_emf<2><<<grid, block, 0, s>>>(g, a.u, a.cell_ez, a.xspd, a.yspd, r, a.gamma, a.ctl); break;
-    case 5: k_cell_emf<5><<<grid, block, 0, s>>>(g, a.u, a.cell_ez, a.xspd, a.yspd, r, a.gamma, a.ctl); break;
-    default: k_cell_emf<7><<<grid, block, 0, s>>>(g, a.u, a.cell_ez, a.xspd, a.yspd, r, a.gamma, a.ctl);
+    case 1: k_cell_emf<1><<<grid, block, 0, s>>>(g, a.u, a.cell_ez, a.xspd, a.yspd, r, a.ctl); break;
+    default: k_cell_emf<2><<<grid, block, 0, s>>>(g, a.u, a.cell_ez, a.xspd, a.yspd, r, a.ctl);
   }
 }
 
