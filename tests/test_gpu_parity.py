@@ -316,7 +316,7 @@ def test_background_queries_on_a_live_solver():
         g.seed_background("b0x", np.zeros(g.grid().storage_size()))
 
 
-def test_preflight_trip_is_the_reference_check():
+def test_preflight_trip_is_the_reference_check(ref):
     """Orszag-Tang 2048^2 MP5: the plain step's live-state solenoidality
     preflight stops the run after about a thousand steps (the smallest grid
     where it trips; 1024^2 reaches t = 0.5).  Running the reference's CPU
@@ -325,7 +325,6 @@ def test_preflight_trip_is_the_reference_check():
     ensure_live_state_solenoidal compares, as a state the solver stepped)
     rejects the state this solver rejected and accepts the last one it
     stepped, against the reference's own tolerance."""
-    ref = M.RefLib()
     if not hasattr(ref.lib, "qref_divb_relative"):
         pytest.skip("reference build without the preflight entry point")
     n, order = 2048, 5
