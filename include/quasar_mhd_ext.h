@@ -36,6 +36,11 @@ int qmhd_probe_roots(const double* x, long long n, double* reciprocal, double* i
  * for checking that the bits are those of IEEE division. */
 int qmhd_probe_quotients(const double* a, const double* b, long long n, double* quotient);
 
+/* The reconstruction's eigen-system (x-normal) of n host states, eight arrays
+ * of n values each: sure[k] is 1 where its bound skips the check of L R = I, and
+ * error[k] the largest entry of |L R - I| of its rows and columns. */
+int qmhd_probe_eigen(const double* states, long long n, double gamma, int* sure, double* error);
+
 /* Tile hooks of a decomposed domain (quasar_b200/tiles.py), the pieces the
  * reference's distributed runtime keeps inside its solver
  * (src/distributed/mhd_runtime.cpp: dt and admissibility reduced over the

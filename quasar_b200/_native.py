@@ -26,7 +26,7 @@ EXPORTS = (
 EXT_EXPORTS = ("qmhd_solver_time_auto_steps", "qmhd_solver_profile_step", "qmhd_fp64_fma_peak",
                "qmhd_conserved_cell_totals_device", "qmhd_solver_set_owned_window",
                "qmhd_solver_write_halo", "qmhd_solver_gather_live", "qmhd_solver_scatter_halo",
-               "qmhd_probe_roots", "qmhd_probe_quotients")
+               "qmhd_probe_roots", "qmhd_probe_quotients", "qmhd_probe_eigen")
 TOTALS_DEVICE_MAX_CELLS = 67108864
 BATCH_EXPORTS = ("qmhd_batch_create", "qmhd_batch_destroy", "qmhd_batch_size", "qmhd_batch_zones",
                  "qmhd_batch_instance", "qmhd_batch_advance", "qmhd_batch_time_steps",
@@ -100,6 +100,7 @@ def lib() -> ctypes.CDLL:
     L.qmhd_fp64_fma_peak.argtypes = [dp]
     L.qmhd_probe_roots.argtypes = [vp, ctypes.c_longlong, vp, vp]
     L.qmhd_probe_quotients.argtypes = [vp, vp, ctypes.c_longlong, vp]
+    L.qmhd_probe_eigen.argtypes = [vp, ctypes.c_longlong, ctypes.c_double, vp, vp]
     L.qmhd_conserved_cell_totals_device.argtypes = [vp, vp, ctypes.c_int, ctypes.c_int,
                                                     ctypes.c_int, vp, dp, dp]
     L.qmhd_batch_create.argtypes = [ctypes.POINTER(QmhdConfig), ctypes.c_int, ctypes.POINTER(vp)]

@@ -334,6 +334,32 @@ int qmhd_probe_quotients(const double* a, const double* b, long long n, double* 
   });
 }
 
+int qmhd_probe_eigen(const double* states, long long n, double gamma, int* sure, double* error) {
+  return guarded([&] {
+    need(states);
+    need(sure);
+    need(error);
+    if (n < 1 || n > (1LL << 24))
+      throw std::invalid_argument("qmhd_probe_eigen: need 1 <= n <= 2^24");
+    if (!(gamma > 1.0)) throw std::invalid_argument("qmhd_probe_eigen: need gamma > 1");
+    struct Buffer {
+      double* p = nullptr;
+      ~Buffer() { cudaFree(p); }
+    } d;
+    const size_t bytes = sizeof(double) * size_t(n);
+    auto ck = [](cudaError_t e) {
+      if (e != cudaSuccess) throw qb::CudaError(std::string("probe_eigen: ") + cudaGetErrorString(e));
+    };
+    ck(cudaMalloc(&d.p, 10 * bytes));
+    int* ds = reinterpret_cast<int*>(d.p + 9 * n);
+    ck(cudaMemcpy(d.p, states, 8 * bytes, cudaMemcpyHostToDevice));
+    qb::launch_probe_eigen(d.p, n, gamma, ds, d.p + 8 * n, nullptr);
+    ck(cudaGetLastError());
+    ck(cudaMemcpy(error, d.p + 8 * n, bytes, cudaMemcpyDeviceToHost));
+    ck(cudaMemcpy(sure, ds, sizeof(int) * size_t(n), cudaMemcpyDeviceToHost));
+  });
+}
+
 // ---- batched instances (include/quasar_mhd_batch.h) ------------------------
 int qmhd_batch_create(const qmhd_config* configs, int n, qmhd_batch** out) {
   return guarded([&] {

@@ -3499,6 +3499,42 @@ __global__ void k_probe_quotients(const double* __restrict__ a, const double* __
   const double v = d.by(b[k]).of(a[k]);
   q[k] = d.bad ? __ddiv_rn(a[k], b[k]) : v;
 }
+// The reconstruction's eigen-system of the states u[0..8)[n] (x-normal): whether
+// its bound skips the L R = I check, and max |L R - I| of the rows and columns it
+// would project with.
+__global__ void k_probe_eigen(const double* __restrict__ u, long long n, double gamma, int* sure,
+                              double* err) {
+  const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const Eg e = eig_scalars(St{u[k], u[n + k], u[2 * n + k], u[3 * n + k], u[4 * n + k], u[5 * n + k],
+                              u[6 * n + k], u[7 * n + k]}, gamma);
+  sure[k] = e.sure;
+  double L[7][7], R[7][7];
+  for (int r = 0; r < 4; ++r) {
+    WavePair w;
+    wave_pair(e, r, w);
+    for (int m = 0; m < 7; ++m) {
+      const double lv = m < 4 && r < 3 ? w.lv[m] : 0.0;
+      const double rv = m > 0 && m < 5 && r < 3 ? w.rv[m - 1] : 0.0;
+      L[r][m] = w.lt[m] - lv;
+      R[r][m] = w.rt[m] - rv;
+      L[6 - r][m] = w.lt[m] + lv;
+      R[6 - r][m] = w.rt[m] + rv;
+    }
+  }
+  double worst = 0.0;
+  for (int a = 0; a < 7; ++a)
+    for (int b = 0; b < 7; ++b) {
+      double s = a == b ? -1.0 : 0.0;
+      for (int m = 0; m < 7; ++m) s = fma(L[a][m], R[b][m], s);
+      worst = fabs(s) <= worst ? worst : fabs(s);  // NaN stays
+    }
+  err[k] = worst;
+}
+void launch_probe_eigen(const double* u, long long n, double gamma, int* sure, double* err,
+                        cudaStream_t s) {
+  if (n > 0) k_probe_eigen<<<cdiv(n, 128), 128, 0, s>>>(u, n, gamma, sure, err);
+}
 void launch_probe_quotients(const double* a, const double* b, long long n, double* q,
                             cudaStream_t s) {
   if (n > 0) k_probe_quotients<<<cdiv(n, 256), 256, 0, s>>>(a, b, n, q);

@@ -320,6 +320,9 @@ void launch_face_lists(const Grid& g, const unsigned char* flag, int* xlist, int
 
 // y[k] and z[k] = the stage kernels' reciprocal and inverse square root of x[k].
 void launch_probe_roots(const double* x, long long n, double* y, double* z, cudaStream_t s);
+// The reconstruction's eigen-systems of n states (eight arrays of n).
+void launch_probe_eigen(const double* u, long long n, double gamma, int* sure, double* err,
+                        cudaStream_t s);
 // q[k] = a[k] / b[k] as the eigen scalars divide.
 void launch_probe_quotients(const double* a, const double* b, long long n, double* q,
                             cudaStream_t s);
