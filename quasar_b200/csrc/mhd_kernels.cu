@@ -1335,7 +1335,7 @@ __device__ __forceinline__ void b_reconstruct(const Grid& g, const StateP& u, co
 // blocks, of both in one launch: the y faces' blocks fill the SMs while the x
 // faces' last ones drain, and a grid that does not fill the chip (a 64^2 grid
 // has 37 blocks a direction) runs both side by side.  64^2 MP5 step 0.26 ->
-// 0.18 ms with the face flux launched the same way.
+// 0.21 ms with the face flux launched the same way.
 template <int ORDER>
 __global__ void __launch_bounds__(128, 4) k_reconstruct(Grid g, StateP u, IfaceP ix, IfaceP iy,
                                                         double gamma, const Ctl* ctl, int dir0) {
