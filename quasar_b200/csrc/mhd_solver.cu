@@ -571,6 +571,7 @@ void MhdSolver2D::advance_positive(double dt) {
   const int prev = last_substeps_;
   if (front_order_ != cfg_.order) front_impl(cfg_.order, 0, -1);
   ++api_steps_;
+  front_order_ = 0;  // the step uses the residual up, and its dt replaces the limit beside it
   if (api_graphs()) {
     *dt_host_ = dt;  // the last step's copy has completed: every step ends with read_ctl
     ck(cudaMemcpyAsync(&ctl_->dt, dt_host_, sizeof(double), cudaMemcpyHostToDevice, stream_), "dt");
@@ -578,7 +579,6 @@ void MhdSolver2D::advance_positive(double dt) {
   } else {
     finish_impl(cfg_.order, nullptr, dt, false);
   }
-  front_order_ = 0;
   const Ctl c = read_ctl();
   if (c.status == 0) {
     promote();

@@ -87,3 +87,13 @@ def test_every_capture_goes_through_it(name):
         text = f.read()
     assert "capture_graphs(" in text
     assert "cudaStreamBeginCapture" not in text and "cudaGraphInstantiate" not in text
+
+
+def test_a_step_gives_up_the_cached_limit_before_it_overwrites_it():
+    """cfl_limit answers from the control block while its residual is cached; a
+    step writes its own dt there, so the cache is dropped first, also when the
+    launch that follows fails."""
+    with open(os.path.join(ROOT, "quasar_b200", "csrc", "mhd_solver.cu")) as f:
+        text = f.read()
+    body = text[text.index("void MhdSolver2D::advance_positive("):text.index("void MhdSolver2D::controller(")]
+    assert body.index("front_order_ = 0;") < body.index("&ctl_->dt, dt_host_")
